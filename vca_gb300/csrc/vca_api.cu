@@ -779,7 +779,7 @@ int sector_gs(int isector, double* E, void** vec_out, Arena& keep) {
       CUCHK(cudaStreamSynchronize(g->st));
       const int kk = mh.len;
       if (kk < 1) { ar.release(); VFAIL(VCA_ERR_NUMERIC, "Lanczos start vector has zero norm"); }
-      launch_tri_lowest(bb.A, bb.Bt, kk, bn, theta, svec, resid, g->st);
+      launch_tri_lowest(bb.A, bb.Bt, kk, bn, c.gs_residual_tol, k == nmax || !mh.active, theta, svec, resid, g->st);
       double rs;
       cudaMemcpyAsync(&th, theta, sizeof(double), cudaMemcpyDeviceToHost, g->st);
       cudaMemcpyAsync(&rs, resid, sizeof(double), cudaMemcpyDeviceToHost, g->st);
@@ -877,7 +877,7 @@ int sector_gs_fx(int isector, double* E, void** vec_out, Arena& keep) {
       CUCHK(cudaStreamSynchronize(g->st));
       const int kk = mh.len;
       if (kk < 1) { ar.release(); VFAIL(VCA_ERR_NUMERIC, "Lanczos start vector has zero norm"); }
-      launch_tri_lowest(bb.A, bb.Bt, kk, bn, theta, svec, resid, g->st);
+      launch_tri_lowest(bb.A, bb.Bt, kk, bn, c.gs_residual_tol, k == nmax || !mh.active, theta, svec, resid, g->st);
       double rs;
       cudaMemcpyAsync(&th, theta, sizeof(double), cudaMemcpyDeviceToHost, g->st);
       cudaMemcpyAsync(&rs, resid, sizeof(double), cudaMemcpyDeviceToHost, g->st);
@@ -995,7 +995,7 @@ int batched_sector_energies(std::vector<double>& energy) {
       ms_launch_step(gp, g->fxs, g->fxbase.K, k, c.gs_beta_tol, b, g->st);
       if (k % std::max(1, c.gs_check_every) == 0 || k == nmaxg) {
         cudaMemsetAsync(b.undone, 0, sizeof(int), g->st);
-        ms_launch_check(gp, b, c.gs_residual_tol, g->st);
+        ms_launch_check(gp, b, c.gs_residual_tol, false, g->st);
         int undone = 0;
         cudaMemcpyAsync(&undone, b.undone, sizeof(int), cudaMemcpyDeviceToHost, g->st);
         CUCHK(cudaStreamSynchronize(g->st));
@@ -1092,7 +1092,7 @@ int batched_sector_energies_f64(std::vector<double>& energy) {
       m64_launch_step(gp, cplx, g->md, k, c.gs_beta_tol, b, g->st);
       if (k % std::max(1, c.gs_check_every) == 0 || k == nmaxg) {
         cudaMemsetAsync(b.undone, 0, sizeof(int), g->st);
-        m64_launch_check(gp, b, c.gs_residual_tol, g->st);
+        m64_launch_check(gp, b, c.gs_residual_tol, false, g->st);
         int undone = 0;
         cudaMemcpyAsync(&undone, b.undone, sizeof(int), cudaMemcpyDeviceToHost, g->st);
         CUCHK(cudaStreamSynchronize(g->st));
@@ -3122,7 +3122,7 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
         m64_launch_step(R.gp, cplx, g->md, k, c.gs_beta_tol, R.b, g->st);
         if (k % std::max(1, c.gs_check_every) == 0 || k == nmaxg) {
           cudaMemsetAsync(R.b.undone, 0, sizeof(int), g->st);
-          m64_launch_check(R.gp, R.b, c.gs_residual_tol, g->st);
+          m64_launch_check(R.gp, R.b, c.gs_residual_tol, true, g->st);
           int undone = 0;
           cudaMemcpyAsync(&undone, R.b.undone, sizeof(int), cudaMemcpyDeviceToHost, g->st);
           if (cudaStreamSynchronize(g->st) != cudaSuccess) { R.ar.release(); VFAIL(VCA_ERR_CUDA, "batched search failed"); }

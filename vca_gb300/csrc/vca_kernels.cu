@@ -474,14 +474,15 @@ void launch_fill(int64_t n, double v, double* X, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // Lowest eigenpair of the Lanczos T_k (one warp, vca_tri.cuh)
 // ---------------------------------------------------------------------------
-__global__ void k_tri_lowest(const double* A, const double* Bt, int k, double btail, double* theta_out,
-                             double* s, double* resid) {
-  warp_tri_lowest(A, Bt, k, btail, theta_out, s, resid);
+__global__ void k_tri_lowest(const double* A, const double* Bt, int k, double btail, double tol, int must_finish,
+                             double* theta_out, double* s, double* resid) {
+  __shared__ float2 w[2 * TRI_MAX];
+  warp_tri_lowest(A, Bt, k, btail, tol, must_finish != 0, true, w, theta_out, s, resid);
 }
-void launch_tri_lowest(const double* A, const double* Bt, int k, double btail, double* theta,
-                       double* s, double* resid, cudaStream_t st) {
+void launch_tri_lowest(const double* A, const double* Bt, int k, double btail, double tol, bool must_finish,
+                       double* theta, double* s, double* resid, cudaStream_t st) {
   COUNT_LAUNCH();
-  k_tri_lowest<<<1, 32, 0, st>>>(A, Bt, k, btail, theta, s, resid);
+  k_tri_lowest<<<1, 32, 0, st>>>(A, Bt, k, btail, tol, must_finish ? 1 : 0, theta, s, resid);
 }
 
 // ---------------------------------------------------------------------------

@@ -72,10 +72,11 @@ void launch_start_vector(int64_t n, uint64_t seed, int isector, double* X, cudaS
 void launch_fill(int64_t n, double v, double* X, cudaStream_t st);
 
 // ---- tridiagonal problems --------------------------------------------------
-// lowest eigenpair of T_k (a[0..k-1], b = beta_{2..k}), residual test;
-// writes theta, s[0..k-1] and flag (1 = converged)
-void launch_tri_lowest(const double* A, const double* Bt, int k, double btail, double* theta,
-                       double* s, double* resid, cudaStream_t st);
+// convergence test of a k-step Lanczos run (warp_tri_lowest, vca_tri.cuh):
+// theta, residual and, where it is converged at tol or must_finish is set, the
+// eigenvector s[0..k-1]
+void launch_tri_lowest(const double* A, const double* Bt, int k, double btail, double tol, bool must_finish,
+                       double* theta, double* s, double* resid, cudaStream_t st);
 // Device store of every Green's function chain: tridiagonal rows A, B
 // ([nch*ld], B[j] = beta_j couples rows j-1 and j), length n, prefactor
 // pes = norm^2*boltz/zeta (boltz = 1 at T=0), isign (+1 particle, -1 hole),

@@ -284,9 +284,11 @@ __global__ void k_ms_record(int nsec, const MsSector* secs, ChainMeta* meta, con
 }
 
 // convergence test of every unfinished sector, one warp per sector
+#define MS_CHECK_WARPS 4
 __global__ void k_ms_check(int nsec, ChainMeta* meta, const double* A, const double* Bt, int ld,
                            const double* bnow, double* svec, double* theta, double* resid, int* state,
-                           int* mconv, double tol, int* undone) {
+                           int* mconv, double tol, int want_vec, int* undone) {
+  __shared__ float2 w[MS_CHECK_WARPS][2 * TRI_MAX];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -298,12 +300,13 @@ __global__ void k_ms_check(int nsec, ChainMeta* meta, const double* A, const dou
       if (lane == 0) { state[s] = 2; theta[s] = INFINITY; mconv[s] = 0; }
       continue;
     }
-    warp_tri_lowest(A + (int64_t)s * ld, Bt + (int64_t)s * ld, kk, bnow[s], theta + s,
-                    svec + (int64_t)s * 5 * ld, resid + s);
-    __syncwarp();
+    const bool full = warp_tri_lowest(A + (int64_t)s * ld, Bt + (int64_t)s * ld, kk, bnow[s], tol, !mt.active,
+                                      want_vec != 0, w[threadIdx.x >> 5], theta + s, svec + (int64_t)s * 5 * ld, resid + s);
     if (lane == 0) {
       const double th = theta[s];
-      if (!mt.active || resid[s] <= tol * fmax(1.0, fabs(th))) {
+      if (!full) {
+        atomicAdd(undone, 1);
+      } else if (!mt.active || resid[s] <= tol * fmax(1.0, fabs(th))) {
         state[s] = 1;
         mconv[s] = kk;
         meta[s].active = 0;
@@ -347,13 +350,13 @@ void ms_launch_step(const MsGroup& gp, const FxScales& fs, int K, int k, double 
   b.X = t;
 }
 
-void ms_launch_check(const MsGroup& gp, MsBufs& b, double tol, cudaStream_t st) {
+void ms_launch_check(const MsGroup& gp, MsBufs& b, double tol, bool want_vec, cudaStream_t st) {
   count_launch_external();
   const int warps = gp.nsec;
-  const int threads = 128;
+  const int threads = 32 * MS_CHECK_WARPS;
   const int blocks = std::max(1, (warps * 32 + threads - 1) / threads);
   k_ms_check<<<blocks, threads, 0, st>>>(gp.nsec, b.meta, b.A, b.Bt, b.ld, b.bnow, b.svec, b.theta, b.resid,
-                                         b.state, b.mconv, tol, b.undone);
+                                         b.state, b.mconv, tol, want_vec ? 1 : 0, b.undone);
 }
 
 
@@ -604,12 +607,12 @@ void m64_launch_step(const MsGroup& gp, bool cplx, const MixedDiag& md, int k, d
   if (cplx) m64_step_t<double2>(gp, md, k, tol, b, st);
   else m64_step_t<double>(gp, md, k, tol, b, st);
 }
-void m64_launch_check(const MsGroup& gp, Ms64Bufs& b, double tol, cudaStream_t st) {
+void m64_launch_check(const MsGroup& gp, Ms64Bufs& b, double tol, bool want_vec, cudaStream_t st) {
   count_launch_external();
-  const int threads = 128;
+  const int threads = 32 * MS_CHECK_WARPS;
   const int blocks = std::max(1, (gp.nsec * 32 + threads - 1) / threads);
   k_ms_check<<<blocks, threads, 0, st>>>(gp.nsec, b.meta, b.A, b.Bt, b.ld, b.bnow, b.svec, b.theta, b.resid,
-                                         b.state, b.mconv, tol, b.undone);
+                                         b.state, b.mconv, tol, want_vec ? 1 : 0, b.undone);
 }
 
 // ---- multi-task helpers of the batched form --------------------------------

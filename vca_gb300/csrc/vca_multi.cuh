@@ -40,7 +40,8 @@ struct MsBufs {
 void ms_launch_start(const MsGroup& gp, uint64_t seed, int F, i64* R, i64* X, i64* tpart, ChainMeta* meta,
                      i64* mul, int* msh, cudaStream_t st);
 void ms_launch_step(const MsGroup& gp, const FxScales& fs, int K, int k, double tol, MsBufs& b, cudaStream_t st);
-void ms_launch_check(const MsGroup& gp, MsBufs& b, double tol, cudaStream_t st);
+// want_vec: the converged tasks' Ritz coefficients into svec too
+void ms_launch_check(const MsGroup& gp, MsBufs& b, double tol, bool want_vec, cudaStream_t st);
 
 // the same search in FP64: vectors of double (real H) or double2 (complex H)
 struct Ms64Bufs {
@@ -54,7 +55,7 @@ struct Ms64Bufs {
 void m64_launch_start(const MsGroup& gp, bool cplx, uint64_t seed, Ms64Bufs& b, cudaStream_t st);
 void m64_launch_step(const MsGroup& gp, bool cplx, const MixedDiag& md, int k, double tol, Ms64Bufs& b,
                      cudaStream_t st);
-void m64_launch_check(const MsGroup& gp, Ms64Bufs& b, double tol, cudaStream_t st);
+void m64_launch_check(const MsGroup& gp, Ms64Bufs& b, double tol, bool want_vec, cudaStream_t st);
 
 // ---- multi-task Lanczos over many variational points (the batched form) --
 // The FP64 step kernels above run any list of tasks: the (point, sector)
