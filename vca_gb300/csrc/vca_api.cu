@@ -25,6 +25,7 @@
 #include "vca_multi.cuh"
 #include "vca_batch.cuh"
 #include "vca_kernels.cuh"
+#include "vca_resident.cuh"
 #include "vca_gfmatrix.h"
 #include "vca_host.h"
 
@@ -156,6 +157,17 @@ struct Ctx {
   int nmax = 0, contour_points = 0;
   std::vector<ChainRec> chains;  // every (element, state, channel)
   int nstore = 0;                // chains in the store, each run once
+  // resident searches of the current diagonalisation (vca_resident.cuh): per
+  // sector its task or -1, and what the vector passes read
+  struct Resident {
+    Arena ar;
+    std::vector<int> slot;
+    std::vector<RsSpace> spaces;
+    std::vector<RsTask> tasks;
+    RsShape shape;
+    void drop() { ar.release(); slot.clear(); spaces.clear(); tasks.clear(); }
+  } rs;
+  int rs_split = 1, rs_diag_im = 0;  // RsParams, of the loaded Hamiltonian
   int ld = 0;
   double* d_poles = nullptr;     // filled on demand from the chain store
   double2* d_weights = nullptr;
@@ -367,6 +379,8 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
     }
   }
   g->real_model = real;
+  g->rs_split = 1;
+  g->rs_diag_im = 0;
   const int LC = c.Nlat * c.Norb;
   for (int set = 0; set < nsets; set++) {
     const int sidx = (set == 0) ? 0 : c.Nspin - 1;
@@ -399,6 +413,8 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
               pairs.push_back({ia, is, v.real(), -v.imag()});
             }
     }
+    for (const HopPair& hp : pairs)
+      if (hp.re != 0.0 && hp.im != 0.0) g->rs_split = 2;
     if ((int)pairs.size() > VCA_MAX_PAIRS) VFAIL(VCA_ERR_UNSUPPORTED, "too many one-body pairs");
     if (set == 0) { g->host_pairs.clear(); g->host_eps_abs.clear(); }
     g->host_pairs.insert(g->host_pairs.end(), pairs.begin(), pairs.end());
@@ -431,6 +447,8 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
           cd e = g->bath_h[idx_bh(c, lb, lb, sidx, sidx, ob, ob)] - c.xmu;
           ep.eps[LC + lb * c.Norb_bath + ob] = make_double2(e.real(), e.imag());
         }
+    for (int l = 0; l < g->Ns; l++)
+      if (ep.eps[l].y != 0.0) g->rs_diag_im = 1;
     {
       double em = 0.0;
       for (int l = 0; l < g->Ns; l++) em = std::max(em, std::abs(cd(ep.eps[l].x, ep.eps[l].y)));
@@ -730,7 +748,11 @@ int alloc_batch(Arena& ar, int64_t rows, int m, bool cplx, int nch, int ldab, Ba
 // Ground state of one sector by Lanczos (replaces SciFortran sp_lanc_eigh,
 // VCA_DIAG.f90:172-184): deterministic start vector, residual test every
 // gs_check_every steps, eigenvector by a second pass over stored coefficients.
+bool resident_sector(int isector);
+int resident_vector(int isector, double* E, void** vec_out, Arena& keep);
+int resident_search(std::vector<double>& energy);
 int sector_gs(int isector, double* E, void** vec_out, Arena& keep) {
+  if (resident_sector(isector)) return resident_vector(isector, E, vec_out, keep);
   const vca_config& c = g->cfg;
   const int nup = sec_nup(isector), ndw = sec_ndw(isector);
   SectorView sv = view_of(nup, ndw);
@@ -828,10 +850,146 @@ int sector_gs(int isector, double* E, void** vec_out, Arena& keep) {
   return VCA_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Resident runs (vca_resident.cuh): searches, eigenvector passes and chains of
+// the sectors whose vectors fit the shared memory of at most RS_MAX_C SMs run
+// whole in one launch.  hxv_variant 1, the comparison arm of the product
+// kernels, keeps the separate launches, and so do two chain streams in fixed
+// point (where both give the same bits).
+// ---------------------------------------------------------------------------
+bool resident_arith() { return (!g->fx || g->fxbase.K <= 2) && g->cfg.hxv_variant != 1; }
+size_t resident_elem() { return g->fx || g->real_model ? sizeof(double) : sizeof(double2); }
+
+RsSpace resident_space(int nup, int ndw) {
+  RsSpace s{};
+  const int du = g->sp[0][nup].dim, dd = g->sp[g->dwset][ndw].dim;
+  s.swap = dd > du ? 1 : 0;
+  s.nat_up = du;
+  s.sv = s.swap ? view_pair(g->dwset, ndw, 0, nup) : view_of(nup, ndw);
+  if (g->fx) {
+    s.fv = s.swap ? fx_view_pair(g->dwset, ndw, 0, nup) : fx_view_of(nup, ndw);
+    s.slow_order = s.swap ? g->fx_perm[0][nup] : g->fx_perm[g->dwset][ndw];
+  }
+  return s;
+}
+RsDims resident_dims(const RsSpace& s, int ncol, int count = 1) {
+  return RsDims{s.sv.dimup, s.sv.dimdw, s.sv.wdw, ncol, count};
+}
+
+int resident_launch(int mode, const std::vector<RsSpace>& spaces, const std::vector<RsTask>& tasks,
+                    const RsShape& shape, Arena& ar) {
+  RsSpace* d_spaces;
+  RsTask* d_tasks;
+  RCHK(ar.alloc(&d_spaces, spaces.size()));
+  RCHK(ar.alloc(&d_tasks, tasks.size()));
+  CUCHK(cudaMemcpyAsync(d_spaces, spaces.data(), sizeof(RsSpace) * spaces.size(), cudaMemcpyHostToDevice, g->st));
+  CUCHK(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(RsTask) * tasks.size(), cudaMemcpyHostToDevice, g->st));
+  RsParams p{};
+  p.spaces = d_spaces;
+  p.tasks = d_tasks;
+  RCHK(ar.alloc(&p.scratch, shape.own * shape.C * tasks.size()));
+  p.scratch_block = shape.own;
+  p.split = g->rs_split;
+  p.diag_im = g->rs_diag_im;
+  p.cs = g->cstore;
+  p.fx = g->fxs;
+  p.md = g->md;
+  p.seed = g->cfg.start_seed;
+  p.beta_tol = mode == RS_CHAIN ? g->cfg.gf_beta_tol : g->cfg.gs_beta_tol;
+  p.resid_tol = g->cfg.gs_residual_tol;
+  p.check_every = std::max(1, g->cfg.gs_check_every);
+  p.mode = mode;
+  if (rs_launch(p, (int)tasks.size(), shape, g->fx ? std::max(1, g->fxbase.K) : 0, !g->real_model, g->st)) CUCHK(cudaGetLastError());
+  CUCHK(cudaGetLastError());
+  return VCA_OK;
+}
+
+// The searches of every sector that fits: energy[] of those sectors, their
+// tasks kept in g->rs for the eigenvector passes.
+int resident_search(std::vector<double>& energy) {
+  const vca_config& c = g->cfg;
+  Ctx::Resident& R = g->rs;
+  R.drop();
+  if (!resident_arith()) return VCA_OK;
+  std::vector<int> order;
+  std::vector<RsDims> dims;
+  R.slot.assign(g->Nsectors + 1, -1);
+  for (int s = 1; s <= g->Nsectors; s++) {
+    const RsSpace sp = resident_space(sec_nup(s), sec_ndw(s));
+    const RsDims d = resident_dims(sp, 1);
+    if (rs_shape(&d, 1, (int)resident_elem(), g->fx, g->rs_split, true).C) order.push_back(s);
+  }
+  auto dim = [&](int s) { return (int64_t)g->dimn[sec_nup(s)] * g->dimn[sec_ndw(s)]; };
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return dim(x) > dim(y); });  // longest first
+  const int n = (int)order.size();
+  if (!n) return VCA_OK;
+  double *theta, *svec;
+  int* mconv;
+  RCHK(R.ar.alloc(&theta, 2 * (size_t)n));
+  RCHK(R.ar.alloc(&svec, (size_t)RS_SVEC * n));
+  RCHK(R.ar.alloc(&mconv, n));
+  for (int i = 0; i < n; i++) {
+    const int s = order[i];
+    R.slot[s] = i;
+    R.spaces.push_back(resident_space(sec_nup(s), sec_ndw(s)));
+    dims.push_back(resident_dims(R.spaces.back(), 1));
+    RsTask t{};
+    t.space = i;
+    t.ncol = 1;
+    t.nlanc = (int)std::min<int64_t>(dim(s), std::min(c.lanc_niter, RS_NMAX));
+    t.isector = s;
+    t.theta = theta + 2 * i;
+    t.svec = svec + (size_t)RS_SVEC * i;
+    t.mconv = mconv + i;
+    R.tasks.push_back(t);
+  }
+  const RsShape shape = rs_shape(dims.data(), dims.size(), (int)resident_elem(), g->fx, g->rs_split, true);
+  if (!shape.C) {
+    R.drop();
+    return VCA_OK;
+  }
+  R.shape = shape;
+  RCHK(resident_launch(RS_SEARCH, R.spaces, R.tasks, shape, R.ar));
+  std::vector<double> th(2 * n);
+  CUCHK(cudaMemcpyAsync(th.data(), theta, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, g->st));
+  CUCHK(cudaStreamSynchronize(g->st));
+  for (int i = 0; i < n; i++) energy[order[i] - 1] = th[2 * i];
+  return VCA_OK;
+}
+bool resident_sector(int isector) {
+  return isector < (int)g->rs.slot.size() && g->rs.slot[isector] >= 0;
+}
+
+// eigenvector of a sector that resident_search ran
+int resident_vector(int isector, double* E, void** vec_out, Arena& keep) {
+  Ctx::Resident& R = g->rs;
+  const RsSpace& sp = R.spaces[R.slot[isector]];
+  RsTask t = R.tasks[R.slot[isector]];
+  const size_t bytes = (size_t)sp.sv.dimup * sp.sv.dimdw * resident_elem();
+  char* psi;
+  RCHK(keep.alloc(&psi, bytes));
+  CUCHK(cudaMemsetAsync(psi, 0, bytes, g->st));
+  t.psi = psi;
+  t.space = 0;
+  // in the search's shape: the pass has to repeat its steps bit for bit, and in
+  // FP64 the order of the sums follows the shape
+  Arena ar;
+  int rc = resident_launch(RS_VECTOR, {sp}, {t}, R.shape, ar);
+  cudaError_t e = cudaMemcpyAsync(E, t.theta, sizeof(double), cudaMemcpyDeviceToHost, g->st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g->st);
+  ar.release();
+  if (rc) return rc;
+  CUCHK(e);
+  if (!std::isfinite(*E)) VFAIL(VCA_ERR_NUMERIC, "Lanczos start vector has zero norm");
+  *vec_out = psi;
+  return VCA_OK;
+}
+
 // Fixed-point variant of sector_gs: same start vector (normalised in FP64,
 // then converted), same stopping rule and second pass; psi stays fixed point
 // (scale 2^-F) for the exact chain gathers.
 int sector_gs_fx(int isector, double* E, void** vec_out, Arena& keep) {
+  if (resident_sector(isector)) return resident_vector(isector, E, vec_out, keep);
   const vca_config& c = g->cfg;
   const FxScales& fs = g->fxs;
   const int nup = sec_nup(isector), ndw = sec_ndw(isector);
@@ -928,6 +1086,7 @@ int batched_sector_energies(std::vector<double>& energy) {
   const vca_config& c = g->cfg;
   const int64_t cap = (int64_t)1 << 28;
   energy.assign(g->Nsectors, INFINITY);
+  RCHK(resident_search(energy));
   int s0 = 1;
   while (s0 <= g->Nsectors) {
     std::vector<MsSector> secs;
@@ -937,6 +1096,7 @@ int batched_sector_energies(std::vector<double>& energy) {
     int nmaxg = 1;
     int s1 = s0;
     while (s1 <= g->Nsectors) {
+      if (resident_sector(s1)) { s1++; continue; }
       const int nu = sec_nup(s1), nd = sec_ndw(s1);
       const int64_t D = (int64_t)g->dimn[nu] * g->dimn[nd];
       if (!secs.empty() && tot + D > cap) break;
@@ -957,6 +1117,7 @@ int batched_sector_energies(std::vector<double>& energy) {
       tot += D;
       s1++;
     }
+    if (secs.empty()) break;  // every sector left ran resident
     const int nsec = (int)secs.size(), ntiles = (int)tsec.size();
     const int ld = nmaxg + 1;
     Arena ar;
@@ -1023,6 +1184,7 @@ int batched_sector_energies_f64(std::vector<double>& energy) {
   const size_t es = cplx ? sizeof(double2) : sizeof(double);
   const int64_t cap = (int64_t)1 << 28;
   energy.assign(g->Nsectors, INFINITY);
+  RCHK(resident_search(energy));
   int s0 = 1;
   while (s0 <= g->Nsectors) {
     std::vector<MsSector> secs;
@@ -1032,6 +1194,7 @@ int batched_sector_energies_f64(std::vector<double>& energy) {
     int nmaxg = 1;
     int s1 = s0;
     while (s1 <= g->Nsectors) {
+      if (resident_sector(s1)) { s1++; continue; }
       const int nu = sec_nup(s1), nd = sec_ndw(s1);
       const int64_t D = (int64_t)g->dimn[nu] * g->dimn[nd];
       if (!secs.empty() && tot + D > cap) break;
@@ -1051,6 +1214,7 @@ int batched_sector_energies_f64(std::vector<double>& energy) {
       tot += D;
       s1++;
     }
+    if (secs.empty()) break;  // every sector left ran resident
     const int nsec = (int)secs.size(), ntiles = (int)tsec.size();
     const int ld = nmaxg + 1;
     Arena ar;
@@ -1461,6 +1625,7 @@ int diagonalize() {
   const vca_config& c = g->cfg;
   g->states.release();
   g->gs.clear();
+  g->rs.drop();
   g->sector_e.assign(g->Nsectors, INFINITY);
   if (c.lanc_method != VCA_LANC_LANCZOS) return g->finiteT ? diagonalize_arpack_finite_t() : diagonalize_arpack_t0();
   if (g->finiteT) return diagonalize_finite_t();
@@ -1569,10 +1734,19 @@ struct ChainKeys {
 // the channels with the index of their chain in specs (ChainRec::store, made
 // absolute once the list has its place in the store).
 struct ChainList {
+  int state = 0, spin = 0;
+  bool dag = false;
+  int base = 0;   // place of specs[0] in the store
   std::vector<ChainSpec> specs;
   std::vector<ChainRec> recs;
   ChainKeys keys;
   int nlanc = 0;  // 0: no target sector
+  bool target(int& tup, int& tdw) const {
+    const int s = g->gs[state].sector, d = dag ? 1 : -1;
+    tup = sec_nup(s) + (spin == 0 ? d : 0);
+    tdw = sec_ndw(s) + (spin == 1 ? d : 0);
+    return tup >= 0 && tup <= g->Ns && tdw >= 0 && tdw <= g->Ns;
+  }
 };
 
 // Boltzmann factor of a state's chains (VCA_GF_NORMAL.f90:987-993): 1 at
@@ -1592,7 +1766,7 @@ struct ChainGroup {
   bool dag = false;
   const std::vector<ChainSpec>* specs = nullptr;
   size_t q0 = 0, q1 = 0;
-  int tup = 0, tdw = 0, m = 0, nch = 0, nlanc = 0;
+  int tup = 0, tdw = 0, m = 0, nch = 0, nlanc = 0, base = 0;
   int64_t D = 0;
   bool swap = false;
   SectorView tv{}, hv{};
@@ -1610,17 +1784,15 @@ struct ChainGroup {
 // Cut the chains of one (state, spin, particle|hole) list into column groups
 // whose three column buffers fit 1/npar of half the free device memory (npar
 // groups run at a time).
-int chain_groups(int state, int spin, bool dag, ChainList& list, int npar, std::vector<ChainGroup>& out) {
+int chain_groups(const ChainList& list, int npar, std::vector<ChainGroup>& out) {
   const std::vector<ChainSpec>& specs = list.specs;
+  const int state = list.state, spin = list.spin;
+  const bool dag = list.dag;
   const vca_config& c = g->cfg;
-  const GState& S = g->gs[state];
-  const int nup = sec_nup(S.sector), ndw = sec_ndw(S.sector);
-  const int tup = nup + (spin == 0 ? (dag ? 1 : -1) : 0);
-  const int tdw = ndw + (spin == 1 ? (dag ? 1 : -1) : 0);
-  if (tup < 0 || tup > g->Ns || tdw < 0 || tdw > g->Ns) return VCA_OK;  // no target sector
+  int tup, tdw;
+  if (!list.target(tup, tdw)) return VCA_OK;
   const SectorView tv = view_of(tup, tdw);
   const int64_t D = (int64_t)tv.dimup * tv.dimdw;
-  list.nlanc = (int)std::min<int64_t>(D, c.lanc_ngfiter);
   const bool cplx = !g->real_model;
   const size_t es = cplx ? sizeof(double2) : sizeof(double);
   size_t freeb = 0, totb = 0;
@@ -1647,6 +1819,7 @@ int chain_groups(int state, int spin, bool dag, ChainList& list, int npar, std::
     G.nch = (int)(q1 - q0);
     G.D = D;
     G.nlanc = list.nlanc;
+    G.base = list.base + (int)q0;
     G.tv = tv;
     out.push_back(G);
     q0 = q1;
@@ -1732,15 +1905,13 @@ int chain_group_step(ChainGroup& G, int k) {
   return lanczos_step(G.tv, G.cb, G.bb, k, c.gf_beta_tol, g->ld, G.st);
 }
 
-// the group's tridiagonals into the chain store, after every earlier group's
+// the group's tridiagonals into the chain store
 int chain_group_finish(ChainGroup& G) {
   const GState& S = g->gs[G.state];
-  const int base = g->nstore;
   launch_chain_store(G.nch, G.bb.meta, G.bb.A, G.bb.Bt, g->ld, G.norm2, G.d_wfac, G.d_isign, S.e, state_weight(S),
-                     g->zeta, g->cstore, base, G.st);
+                     g->zeta, g->cstore, G.base, G.st);
   CUCHK(cudaGetLastError());
   CUCHK(cudaStreamSynchronize(G.st));
-  g->nstore += G.nch;
   G.ar.release();
   return VCA_OK;
 }
@@ -1778,6 +1949,79 @@ int run_chain_groups(std::vector<ChainGroup>& groups, int npar) {
     g->chain_ms[1] += now_ms() - tb1;
     g->chain_ms[2] += (double)(j1 - i);
   }
+  return VCA_OK;
+}
+
+// The lists whose target sectors fit: every chain in one launch, straight
+// into the chain store.  ran[i]: list i is done.
+int resident_chains(const std::vector<ChainList>& lists, std::vector<char>& ran) {
+  ran.assign(lists.size(), 0);
+  if (!resident_arith() || (g->fx && g->chain_streams > 1)) return VCA_OK;
+  const double t0 = now_ms();
+  const int es = (int)resident_elem();
+  std::vector<RsSpace> spaces;
+  std::vector<RsTask> tasks;
+  std::vector<RsDims> dims;
+  int nlists = 0;
+  for (size_t i = 0; i < lists.size(); i++) {
+    const ChainList& v = lists[i];
+    int tup, tdw;
+    if (!v.nlanc || !v.target(tup, tdw)) continue;
+    const RsSpace sp = resident_space(tup, tdw);
+    int two = 0;
+    for (const ChainSpec& q : v.specs) two += q.ncol == 2;
+    const RsDims d[2] = {resident_dims(sp, 1, (int)v.specs.size() - two), resident_dims(sp, 2, two)};
+    if (!rs_shape(d, two ? 2 : 1, es, g->fx, g->rs_split, false).C) continue;
+    dims.insert(dims.end(), d, d + (two ? 2 : 1));
+    if (!rs_shape(dims.data(), dims.size(), es, g->fx, g->rs_split, false).C) {  // not in one launch with the lists before it
+      dims.resize(dims.size() - (two ? 2 : 1));
+      continue;
+    }
+    ran[i] = 1;
+    nlists++;
+    const GState& S = g->gs[v.state];
+    const int nup = sec_nup(S.sector), ndw = sec_ndw(S.sector), nsrc = v.spin == 0 ? nup : ndw;
+    spaces.push_back(sp);
+    for (size_t q = 0; q < v.specs.size(); q++) {
+      const ChainSpec& c = v.specs[q];
+      RsTask t{};
+      t.space = (int)spaces.size() - 1;
+      t.ncol = c.ncol;
+      t.nlanc = v.nlanc;
+      t.gs = S.vec;
+      t.src_words = g->words[nsrc];
+      t.src_dim = g->dimn[nsrc];
+      t.src_dimup = g->sp[0][nup].dim;
+      t.spin = c.ci.spin;
+      t.dag = c.ci.dag;
+      t.nterm = c.ci.nterm;
+      for (int x = 0; x < 2; x++) {
+        t.pos[x] = c.ci.t[x].pos;
+        t.cre[x] = (int)c.ci.t[x].re;
+        t.cim[x] = (int)c.ci.t[x].im;
+      }
+      t.boltz = state_weight(S);
+      t.zeta = g->zeta;
+      t.Ei = S.e;
+      t.isign = c.isign;
+      t.wfac = make_double2(c.wfac.real(), c.wfac.imag());
+      t.store = v.base + (int)q;
+      tasks.push_back(t);
+    }
+  }
+  if (tasks.empty()) return VCA_OK;
+  std::stable_sort(tasks.begin(), tasks.end(), [&](const RsTask& a, const RsTask& b) {  // longest first
+    const SectorView &x = spaces[a.space].sv, &y = spaces[b.space].sv;
+    return (int64_t)a.ncol * x.dimup * x.dimdw > (int64_t)b.ncol * y.dimup * y.dimdw;
+  });
+  Arena ar;
+  int rc = resident_launch(RS_CHAIN, spaces, tasks, rs_shape(dims.data(), dims.size(), es, g->fx, g->rs_split, false), ar);
+  const cudaError_t e = cudaStreamSynchronize(g->st);
+  ar.release();
+  if (rc) return rc;
+  CUCHK(e);
+  g->chain_ms[1] += now_ms() - t0;
+  g->chain_ms[2] += nlists;
   return VCA_OK;
 }
 
@@ -1838,6 +2082,9 @@ int build_gf() {
       speclists.emplace_back();
       ChainList& hole = speclists.back();
       part.keys.cplx = hole.keys.cplx = cplx;
+      part.state = hole.state = k;
+      part.spin = hole.spin = is;
+      part.dag = true;
       auto add = [&](ChainList& v, int dag, int e, int chan, int p, cd cp, int q, cd cq,
                      int nterm, cd wfac) {
         ChainSpec s{};
@@ -1874,20 +2121,24 @@ int build_gf() {
               }
             }
         }
-      RCHK(chain_groups(k, is, true, part, npar, groups));
-      RCHK(chain_groups(k, is, false, hole, npar, groups));
     }
-  RCHK(run_chain_groups(groups, npar));
-  int base = 0;
-  for (const ChainList& v : speclists) {
-    if (!v.nlanc) continue;
+  for (ChainList& v : speclists) {
+    int tup, tdw;
+    if (!v.target(tup, tdw)) continue;
+    v.nlanc = (int)std::min<int64_t>((int64_t)g->dimn[tup] * g->dimn[tdw], c.lanc_ngfiter);
+    v.base = g->nstore;
+    g->nstore += (int)v.specs.size();
     for (ChainRec r : v.recs) {
       r.nlanc = v.nlanc;
-      r.store += base;
+      r.store += v.base;
       g->chains.push_back(r);
     }
-    base += (int)v.specs.size();
   }
+  std::vector<char> ran;
+  RCHK(resident_chains(speclists, ran));
+  for (size_t i = 0; i < speclists.size(); i++)
+    if (!ran[i]) RCHK(chain_groups(speclists[i], npar, groups));
+  if (!groups.empty()) RCHK(run_chain_groups(groups, npar));
   std::vector<int> ptr, flat;
   element_chains(ptr, flat);
   RCHK(g->gf.alloc(&g->d_elem_ptr, ptr.size()));
@@ -3559,6 +3810,7 @@ int vca_gpu_finalize(void) {
   g->states.release();
   g->ham.release();
   g->basis.release();
+  g->rs.drop();
   if (g->st) cudaStreamDestroy(g->st);
   if (g->st2) cudaStreamDestroy(g->st2);
   delete g;
