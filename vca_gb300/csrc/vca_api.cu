@@ -2192,8 +2192,15 @@ int gf_lso(int nz, const double2* d_z, double2* d_Glso, Arena& ar, bool solve_ta
   RCHK(ar.alloc(&raw, (size_t)nz * nelem));
   if (g->gfm_loaded && !solve_tables)
     launch_gf_eval_poles(nelem, g->d_gfm_ptr, g->d_gfm_p, g->d_gfm_w, nz, d_z, raw, g->st);
-  else
-    launch_gf_eval(gf_layout(), nz, d_z, raw, g->st);
+  else {
+    // in runs of points whose chain values take at most 256 MB
+    const int nch = g->nstore;
+    const int most = (int)std::max<int64_t>(1, std::min<int64_t>(nz, ((int64_t)1 << 24) / std::max(1, nch)));
+    double2* val;
+    RCHK(ar.alloc(&val, (size_t)most * nch));
+    for (int q = 0; q < nz; q += most)
+      launch_gf_eval(gf_layout(), nch, std::min(most, nz - q), d_z + q, val, raw + (size_t)q * nelem, g->st);
+  }
   ClusterDims cdm{c.Nlat, c.Norb, c.Nspin, g->N, c.vca_gf_symmetric ? 0 : 1};
   launch_gf_assemble(cdm, nz, raw, d_Glso, g->st);
   CUCHK(cudaGetLastError());
@@ -2391,8 +2398,25 @@ int ksum_device(int n, const double2* d_z, bool want_im, Arena& ar, double** f_r
     ki.ldG = ldG;
     ki.omega_c = 10.0;
   }
-  launch_omega_ksum2(n, N, nblk, nb, P, Glso, nks, hks, pairs ? g->d_kw : nullptr, d_rowptr, d_cols, fpart,
-                     fpart_im, kchunks, pre_m, ki, g->st);
+  const int nq = (int)cols.size();
+  const double* kw = pairs ? g->d_kw : nullptr;
+  if (!want_im && ksum_lu_ok(N, nblk, nb, nq, pre_m)) {
+    std::vector<int> pat(2 * (size_t)nq);  // lso element index; row | col << 8 within the block
+    for (int a = 0; a < N; a++)
+      for (int q = rowptr[a]; q < rowptr[a + 1]; q++) {
+        pat[q] = a + cols[q] * N;
+        pat[nq + q] = a % nb | (cols[q] % nb) << 8;
+      }
+    int* d_pat;
+    double2* Mt;
+    if ((rc = ar.alloc(&d_pat, pat.size())) || (rc = ar.alloc(&Mt, (size_t)nq * nks))) return rc;
+    if (nq) CUCHK(cudaMemcpyAsync(d_pat, pat.data(), sizeof(int) * pat.size(), cudaMemcpyHostToDevice, g->st));
+    launch_ksum_lu(n, N, nblk, nb, nq, d_pat, d_pat + nq, d_rowptr, P, Glso, nks, hks, Mt, kw, fpart, kchunks, pre_m,
+                   ki, g->st);
+  } else {
+    launch_omega_ksum2(n, N, nblk, nb, P, Glso, nks, hks, kw, d_rowptr, d_cols, fpart, fpart_im, kchunks, pre_m, ki,
+                       g->st);
+  }
   launch_reduce_rows(n, kchunks, fpart, 1.0 / (double)Nk, *f_re, g->st);
   if (want_im) launch_reduce_rows(n, kchunks, fpart_im, 1.0 / (double)Nk, *f_im, g->st);
   CUCHK(cudaGetLastError());

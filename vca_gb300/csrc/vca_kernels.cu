@@ -752,52 +752,105 @@ void launch_chain_init(const SectorView& tgt, int src_dimup, const void* gs, boo
   }
 }
 
-// ---------------------------------------------------------------------------
-// Cluster Green's function from poles (vca_gf_cluster_scalar,
-// VCA_IO/gf_cluster.f90:23-49) and recombination (:50-62).
-// ---------------------------------------------------------------------------
-// Per (z, element) thread: sum over the element's chains of
+// Raw element sums of the chains (vca_gf_cluster's sum over states and
+// channels).  A chain's value at z is
 // isign * pes * wfac / (zeta' - a0 - b1^2 / (zeta' - a1 - ...)), zeta' =
 // isign*z + Ei: the continued fraction of the chain's tridiagonal, equal to
 // the sum over its poles isign*(E_j - Ei) with weights wfac*pes*Z(1,j)^2.
-__global__ void k_gf_eval(GfLayout g, int nz, const double2* z, double2* G) {
+//
+// The fractions are bound by the FP64 pipe, so each chain is evaluated once
+// per z (k_chain_eval) although several elements sum it (k_gf_sum), b^2 comes
+// squared from shared memory, and the quotient b^2 / |t|^2 is the product with
+// a reciprocal from an FP32 estimate and one cubic Newton step (4 FP64
+// operations; relative error 2^-66 before its rounding) while |t|^2 is in
+// FP32's range: 10 FP64 operations a row, 17 with the division.
+// 3x2 cluster, 8,000 points: 11.7 -> 5.8 ms; BHZ, 8192 evaluations: 10.9 -> 7.7 ms.
+#define GF_ROWS 256  // rows of a chain staged at a time
+__device__ __forceinline__ double gf_recip(double d) {
+  if (d > 1e-30 && d < 1e30) {
+    const double g = (double)__frcp_rn((float)d);
+    const double e = fma(-d, g, 1.0);
+    return fma(g, fma(e, e, e), g);
+  }
+  return 1.0 / d;
+}
+__global__ void __launch_bounds__(128) k_chain_eval(ChainStore cs, int nz, const double2* z, double2* val) {
+  __shared__ double2 ab[GF_ROWS];
+  const int ch = blockIdx.y;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int np = cs.n[ch];
+  const double sg = (double)cs.isign[ch];
+  const double* A = cs.A + (int64_t)ch * cs.ld;
+  const double* B = cs.B + (int64_t)ch * cs.ld;
+  double zr = 0.0, zi = 0.0;
+  if (q < nz) {
+    zr = sg * z[q].x + cs.Ei[ch];
+    zi = sg * z[q].y;
+  }
+  // t starts above the last row: b = 0 there
+  double tr = 1.0, ti = 0.0;
+  for (int r1 = np; r1 > 0; r1 -= GF_ROWS) {
+    const int r0 = max(0, r1 - GF_ROWS);
+    __syncthreads();
+    for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+      const double b = r + 1 < np ? B[r + 1] : 0.0;
+      ab[r - r0] = make_double2(A[r], b * b);
+    }
+    __syncthreads();
+    if (q < nz) {
+#pragma unroll 2
+      for (int r = r1 - 1 - r0; r >= 0; r--) {
+        const double2 x = ab[r];
+        const double inv = x.y * gf_recip(fma(tr, tr, ti * ti));  // b^2 / t = b^2 conj(t) / |t|^2
+        tr = fma(-tr, inv, zr - x.x);
+        ti = fma(ti, inv, zi);
+      }
+    }
+  }
+  if (q >= nz) return;
+  double2 out = make_double2(0.0, 0.0);
+  if (np > 0) {
+    const double inv = 1.0 / fma(tr, tr, ti * ti);
+    const double cr = tr * inv, ci = -ti * inv;
+    const double f = sg * cs.pes[ch];
+    const double2 w = cs.wfac[ch];
+    const double wr = w.x * f, wi = w.y * f;
+    out = make_double2(wr * cr - wi * ci, wr * ci + wi * cr);
+  }
+  val[(int64_t)ch * nz + q] = out;
+}
+__global__ void k_gf_sum(GfLayout g, int nz, const double2* val, double2* G) {
   const int64_t n = (int64_t)nz * g.nelem;
-  const ChainStore& cs = g.cs;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x) {
     const int e = (int)(t % g.nelem);
     const int q = (int)(t / g.nelem);
     double ar = 0.0, ai = 0.0;
     for (int x = g.elem_ptr[e]; x < g.elem_ptr[e + 1]; x++) {
-      const int ch = g.elem_chain[x];
-      const int np = cs.n[ch];
-      if (np <= 0) continue;
-      const double sg = (double)cs.isign[ch];
-      const double zr = sg * z[q].x + cs.Ei[ch], zi = sg * z[q].y;
-      const double* A = cs.A + (int64_t)ch * cs.ld;
-      const double* B = cs.B + (int64_t)ch * cs.ld;
-      double tr = zr - A[np - 1], ti = zi;
-      for (int k = np - 2; k >= 0; k--) {
-        const double b2 = B[k + 1] * B[k + 1];
-        const double inv = b2 / fma(tr, tr, ti * ti);  // b^2 / t = b^2 conj(t) / |t|^2
-        tr = zr - A[k] - tr * inv;
-        ti = zi + ti * inv;
-      }
-      const double inv = 1.0 / fma(tr, tr, ti * ti);
-      const double cr = tr * inv, ci = -ti * inv;
-      const double f = sg * cs.pes[ch];
-      const double2 w = cs.wfac[ch];
-      const double wr = w.x * f, wi = w.y * f;
-      ar += wr * cr - wi * ci;
-      ai += wr * ci + wi * cr;
+      const double2 v = val[(int64_t)g.elem_chain[x] * nz + q];
+      ar += v.x;
+      ai += v.y;
     }
     G[t] = make_double2(ar, ai);
   }
 }
-void launch_gf_eval(const GfLayout& g, int nz, const double2* z, double2* G, cudaStream_t st) {
+void launch_gf_eval(const GfLayout& g, int nch, int nz, const double2* z, double2* val, double2* G, cudaStream_t st) {
+  if (nz <= 0) return;
+  for (int c0 = 0; c0 < nch; c0 += 65535) {  // grid.y limit
+    const int n = std::min(nch - c0, 65535);
+    ChainStore cs = g.cs;
+    cs.A += (int64_t)c0 * cs.ld;
+    cs.B += (int64_t)c0 * cs.ld;
+    cs.n += c0;
+    cs.pes += c0;
+    cs.isign += c0;
+    cs.wfac += c0;
+    cs.Ei += c0;
+    COUNT_LAUNCH();
+    k_chain_eval<<<dim3((nz + 127) / 128, n), 128, 0, st>>>(cs, nz, z, val + (int64_t)c0 * nz);
+  }
   COUNT_LAUNCH();
-  int64_t n = (int64_t)nz * g.nelem;
-  k_gf_eval<<<nblocks(n, 128), 128, 0, st>>>(g, nz, z, G);
+  k_gf_sum<<<nblocks((int64_t)nz * g.nelem, 128), 128, 0, st>>>(g, nz, val, G);
 }
 
 // Pole tables as vca_gf_cluster_scalar sums them (VCA_IO/gf_cluster.f90:
@@ -1584,6 +1637,312 @@ void launch_omega_ksum2(int nw, int N, int nblk, int nb, const double2* P, const
   else
     ksum2_dispatch<false>(nw, N, nblk, nb, P, Glso, Nk, Hk, kw, rowptr, cols, fpart, nullptr, kchunks, pre_m, ki,
                           st);
+}
+
+// ---------------------------------------------------------------------------
+// The T=0 integrand for blocks up to KLU_MAX: whole determinants per thread.
+//
+// A determinant of an 8 x 8 block is ~900 FP64 operations, and the lane-group
+// form above spends 3 times the warp instructions that makes: the pivots'
+// reciprocals run on one lane of eight and its short updates leave lanes
+// idle.  Here L lanes (klu_shape) own a matrix, stored [element][matrix] in
+// shared memory so that a warp's accesses are contiguous, and every lane of a warp
+// does the same work on another k:
+//  * M = P - H_k comes transposed, [pattern entry][k], so a warp reads it
+//    coalesced;
+//  * pivots are compared by the high words of |re|, |im| (any row near the
+//    largest keeps the elimination stable), their reciprocals are an FP32
+//    estimate and one cubic Newton step (gf_recip);
+//  * the pivots' squared moduli are multiplied up over all k of a thread, as
+//    mantissa and exponent, and so are the 1 + delta of the unpivoted form: a
+//    thread takes a few logarithms at its end instead of one a determinant.
+// FP64-pipe bound.  BHZ 2x2 (2304 k, 4096 nodes, two 8 x 8 blocks): 121.3 ->
+// 46.1 ms; 4x3 (514 k, 8192 nodes, 12 x 12): 53.4 -> 34.7 ms.
+// ---------------------------------------------------------------------------
+#define KLU_MAX 20
+#define KLU_SMEM (226 * 1024)
+#define KLU_T 96  // most threads
+
+// transposed pattern entries: out[q*nks + k] = src[k*NN + il[q]]
+__global__ void k_pattern_t(int64_t nks, int NN, int nq, const int* il, const double2* src, double2* out) {
+  const int64_t n = nks * nq;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t q = t / nks, k = t - q * nks;
+    out[t] = src[k * NN + il[q]];
+  }
+}
+
+struct KluProd {  // prod as mantissa in [1, 2) and exponent
+  double m = 1.0;
+  int e = 0;
+  __device__ __forceinline__ void mul(double x) {
+    m *= x;
+    const int hi = __double2hiint(m), ex = ((hi >> 20) & 2047) - 1023;
+    e += ex;
+    m = __hiloint2double(hi - (ex << 20), __double2loint(m));
+  }
+  __device__ __forceinline__ double log_() const { return log(m) + e * 0.6931471805599453; }
+};
+
+template <int L>
+__global__ void __launch_bounds__(KLU_T) k_ksum_lu(int N, int nblk, int nb, int nq, const int* ent, const int* rowptr,
+                                                 const double2* P, const double2* Glso, int64_t nks,
+                                                 const double2* Mt, const double* kw, double* fpart, int kchunks,
+                                                 int pre_m, const double2* zn, const double2* Ginv, const double* ldG,
+                                                 double omega_c) {
+  constexpr int WM = 32 / L;
+  const int MT = (int)blockDim.x / L;
+  extern __shared__ double2 shm[];
+  const int w = blockIdx.y, chunk = blockIdx.x, NN = N * N, nbb = nb * nb;
+  double2* A = shm;                  // [nbb][MT]
+  double2* Gs = A + (size_t)nbb * MT;  // [nblk][nbb]
+  double2* Pe = Gs + nblk * nbb;     // [nq], when P depends on the node
+  int* es = (int*)(Pe + (pre_m ? 0 : nq));  // row | col << 8 within the block
+  int* rp = es + nq;                 // [N + 1]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slot = warp * WM + lane % WM, part = lane / WM;
+  const bool inv = Ginv != nullptr && zn[w].y <= omega_c;  // as k_omega_ksum2
+  const double2* Gsrc = (inv ? Ginv : Glso) + (int64_t)w * NN;
+  for (int t = threadIdx.x; t < nblk * nbb; t += blockDim.x) {
+    const int b = t / nbb, r = t - b * nbb, i = r % nb, j = r / nb;
+    Gs[t] = Gsrc[(b * nb + i) + (int64_t)(b * nb + j) * N];
+  }
+  for (int t = threadIdx.x; t < nq; t += blockDim.x) es[t] = ent[t];
+  for (int t = threadIdx.x; t <= N; t += blockDim.x) rp[t] = rowptr[t];
+  __syncthreads();
+  if (!pre_m)
+    for (int a = threadIdx.x; a < N; a += blockDim.x)
+      for (int q = rp[a]; q < rp[a + 1]; q++)
+        Pe[q] = P[(int64_t)w * NN + a + (int64_t)((a / nb) * nb + (es[q] >> 8)) * N];
+  __syncthreads();
+  const int64_t k0 = (nks * chunk) / kchunks, k1 = (nks * (chunk + 1)) / kchunks;
+  const int nk = (int)(k1 - k0), ntask = nk * nblk;
+  double2* a0 = A + slot;
+#define KA(i, j) a0[((i) + (j) * nb) * MT]
+  double acc = 0.0, d1 = 0.0, d2 = 0.0;
+  KluProd p1, p2;
+  for (int it = slot; it - slot < ntask; it += MT) {
+    const bool valid = it < ntask;
+    const int t = valid ? it : ntask - 1;
+    const int b = t / nk;
+    const int64_t k = k0 + (t - b * nk);
+    const double2* g = Gs + b * nbb;
+    const double2* mk = Mt + k;
+    auto entry = [&](int q) {
+      double2 m = mk[(int64_t)q * nks];
+      if (!pre_m) m = make_double2(Pe[q].x - m.x, Pe[q].y - m.y);
+      return m;
+    };
+    bool small = false;
+    if (inv) {  // G^-1 + M
+      for (int j = part; j < nb; j += L)
+        for (int i = 0; i < nb; i++) KA(i, j) = g[i + j * nb];
+      for (int q = rp[b * nb]; q < rp[(b + 1) * nb]; q++) {
+        const int i = es[q] & 255, j = es[q] >> 8;
+        if (L > 1 && j % L != part) continue;
+        const double2 m = entry(q), x = KA(i, j);
+        KA(i, j) = make_double2(x.x + m.x, x.y + m.y);
+      }
+    } else {  // M G, four columns at a time
+      for (int jc = part; jc < nb; jc += 4 * L)
+        for (int i = 0; i < nb; i++) {
+          double2 s[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++) s[c] = make_double2(0.0, 0.0);
+          for (int q = rp[b * nb + i]; q < rp[b * nb + i + 1]; q++) {
+            const double2 m = entry(q);
+            const double2* gr = g + (es[q] >> 8);
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+              if (jc + c * L < nb) {
+                const double2 x = gr[(jc + c * L) * nb];
+                s[c].x = fma(m.x, x.x, s[c].x);
+                s[c].x = fma(-m.y, x.y, s[c].x);
+                s[c].y = fma(m.x, x.y, s[c].y);
+                s[c].y = fma(m.y, x.x, s[c].y);
+              }
+          }
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+            if (jc + c * L < nb) KA(i, jc + c * L) = s[c];
+        }
+      if (L > 1) __syncwarp();
+      // elimination without pivoting while the row sums of |re| + |im| stay below 1/2
+      double rmax = 0.0;
+      for (int i = 0; i < nb; i++) {
+        double r = 0.0;
+        for (int j = 0; j < nb; j++) {
+          const double2 x = KA(i, j);
+          r += fabs(x.x) + fabs(x.y);
+        }
+        rmax = fmax(rmax, r);
+      }
+      small = rmax < 0.49;
+      if (L > 1) __syncwarp();
+      if (!small)
+        for (int j = part; j < nb; j += L) KA(j, j).x += 1.0;
+    }
+    if (L > 1) __syncwarp();
+    KluProd pt;
+    double delta = 0.0, odd = 0.0;
+    bool zero = false;
+    for (int kk = 0; kk < nb; kk++) {
+      int arg = kk;
+      double2 piv;
+      if (small) {
+        const double2 x = KA(kk, kk);
+        const double u = fma(x.x, x.x, fma(x.y, x.y, 2.0 * x.x));
+        delta = delta + u + delta * u;
+        piv = make_double2(1.0 + x.x, x.y);
+      } else {
+        int best = -1;
+        for (int i = kk; i < nb; i++) {
+          const double2 x = KA(i, kk);
+          const int h = max(__double2hiint(x.x) & 0x7fffffff, __double2hiint(x.y) & 0x7fffffff);
+          if (h > best) { best = h; arg = i; }
+        }
+        piv = KA(arg, kk);
+      }
+      const double mag = fma(piv.x, piv.x, piv.y * piv.y);
+      if (!small) {
+        if (mag < 2.2250738585072014e-308) zero = true;  // |pivot| below 1e-154: treated as singular
+        else if (mag < 1e300) pt.mul(mag);
+        else odd += log(mag);  // out of the product's range, infinite or NaN
+      }
+      if (L > 1) __syncwarp();
+      if (arg != kk)
+        for (int j = kk + (part - kk % L + L) % L; j < nb; j += L) {
+          const double2 x = KA(kk, j), y = KA(arg, j);
+          KA(kk, j) = y;
+          KA(arg, j) = x;
+        }
+      if (L > 1) __syncwarp();
+      const double rg = gf_recip(mag), ir = piv.x * rg, ii = -piv.y * rg;
+      for (int j = kk + 1 + (part - (kk + 1) % L + L) % L; j < nb; j += 2 * L) {  // two own columns at a time
+        const bool two = j + L < nb;
+        const double2 x = KA(kk, j), y = two ? KA(kk, j + L) : make_double2(0.0, 0.0);
+        const double2 u = make_double2(x.x * ir - x.y * ii, x.x * ii + x.y * ir);
+        const double2 v = make_double2(y.x * ir - y.y * ii, y.x * ii + y.y * ir);
+#pragma unroll 2
+        for (int i = kk + 1; i < nb; i++) {
+          const double2 l = KA(i, kk);
+          double2 s = KA(i, j);
+          s.x = fma(-l.x, u.x, s.x);
+          s.y = fma(-l.x, u.y, s.y);
+          s.x = fma(l.y, u.y, s.x);
+          s.y = fma(-l.y, u.x, s.y);
+          KA(i, j) = s;
+          if (two) {
+            double2 r = KA(i, j + L);
+            r.x = fma(-l.x, v.x, r.x);
+            r.y = fma(-l.x, v.y, r.y);
+            r.x = fma(l.y, v.y, r.x);
+            r.y = fma(-l.y, v.x, r.y);
+            KA(i, j + L) = r;
+          }
+        }
+      }
+      if (L > 1) __syncwarp();
+    }
+    if (valid && part == 0) {
+      const double wt = kw ? kw[k] : 1.0;
+      if (inv) acc = fma(wt, ldG[(int64_t)w * nblk + b], acc);
+      acc = fma(wt, 0.5 * odd, acc);
+      if (zero) {
+        acc = -INFINITY;
+      } else if (wt == 1.0) {
+        if (small) d1 = d1 + delta + d1 * delta; else { p1.mul(pt.m); p1.e += pt.e; }
+      } else if (wt == 2.0) {
+        if (small) d2 = d2 + delta + d2 * delta; else { p2.mul(pt.m); p2.e += pt.e; }
+      } else {
+        acc = fma(wt, 0.5 * (small ? log1p(delta) : pt.log_()), acc);
+      }
+    }
+    if (L > 1) __syncwarp();
+  }
+#undef KA
+  acc += 0.5 * (p1.log_() + log1p(d1)) + (p2.log_() + log1p(d2));
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  __shared__ double red[KLU_T / 32];
+  if (lane == 0) red[warp] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int i = 0; i < (int)blockDim.x / 32; i++) s += red[i];
+    fpart[(int64_t)w * kchunks + chunk] = s;
+  }
+}
+
+// Launch shape: a warp's 32 / L matrices take 512 nb^2 / L bytes, and about
+// five warps an SM keep the FP64 pipe busy across one another's pivot
+// searches and reciprocals (8 x 8 blocks: 59 ms with 4 warps, 45 with 6), so
+// the fewest lanes a matrix that leave five, and the block size that packs
+// the most of them.  More lanes repeat the pivots' scalars: 8 x 8 with two
+// lanes 61 ms, 12 x 12 with one, two, four lanes 44, 35, 42 ms.
+struct KluShape {
+  int L = 0, T = 0;
+  size_t smem = 0;
+};
+static KluShape klu_shape(int N, int nblk, int nb, int nq, bool pre_m) {
+  KluShape best;
+  int most = 0;
+  for (int L = 1; L <= 4 && most < 5; L *= 2)
+    for (int T = KLU_T; T >= 32; T -= 32) {
+      const size_t b = sizeof(double2) * ((size_t)nb * nb * (T / L) + (size_t)nblk * nb * nb + (pre_m ? 0 : nq)) +
+                       sizeof(int) * (size_t)(nq + N + 1);
+      const int warps = b > KLU_SMEM ? 0 : (int)std::min<size_t>(16, KLU_SMEM / (b + 1024) * (T / 32));
+      if (warps > most || (warps && !most)) {
+        most = warps;
+        best.L = L;
+        best.T = T;
+        best.smem = b;
+      }
+    }
+  return best;
+}
+bool ksum_lu_ok(int N, int nblk, int nb, int nq, bool pre_m) {
+  return nb <= KLU_MAX && klu_shape(N, nblk, nb, nq, pre_m).L > 0;
+}
+template <int L>
+static void ksum_lu_go(int nw, int N, int nblk, int nb, int nq, const int* ent, const int* rowptr, const double2* P,
+                       const double2* Glso, int64_t nks, const double2* Mt, const double* kw, double* fpart,
+                       int kchunks, bool pre_m, const KsumInverse& ki, const KluShape& sh, cudaStream_t st) {
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_ksum_lu<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, KLU_SMEM);
+    attr = true;
+  }
+  k_ksum_lu<L><<<dim3(kchunks, nw, 1), sh.T, sh.smem, st>>>(
+      N, nblk, nb, nq, ent, rowptr, P, Glso, nks, Mt, kw, fpart, kchunks, pre_m ? 1 : 0, ki.z, ki.Ginv, ki.ldG,
+      ki.omega_c);
+}
+void launch_ksum_lu(int nw, int N, int nblk, int nb, int nq, const int* il, const int* ent, const int* rowptr,
+                    const double2* P, const double2* Glso, int64_t nks, const double2* M, double2* Mt,
+                    const double* kw, double* fpart, int kchunks, bool pre_m, const KsumInverse& ki,
+                    cudaStream_t st) {
+  if (nq > 0) {
+    COUNT_LAUNCH();
+    k_pattern_t<<<nblocks(nks * nq, 256), 256, 0, st>>>(nks, N * N, nq, il, M, Mt);
+  }
+  const KluShape sh = klu_shape(N, nblk, nb, nq, pre_m);
+  for (int w0 = 0; w0 < nw; w0 += 65535) {  // grid.y limit
+    const int n = std::min(nw - w0, 65535);
+    const int64_t o = (int64_t)w0 * N * N;
+    KsumInverse k2 = ki;
+    if (ki.Ginv) {
+      k2.z += w0;
+      k2.Ginv += o;
+      k2.ldG += (int64_t)w0 * nblk;
+    }
+    COUNT_LAUNCH();
+    const double2* Pw = pre_m ? P : P + o;
+    double* fp = fpart + (int64_t)w0 * kchunks;
+    switch (sh.L) {
+      case 1: ksum_lu_go<1>(n, N, nblk, nb, nq, ent, rowptr, Pw, Glso + o, nks, Mt, kw, fp, kchunks, pre_m, k2, sh, st); break;
+      case 2: ksum_lu_go<2>(n, N, nblk, nb, nq, ent, rowptr, Pw, Glso + o, nks, Mt, kw, fp, kchunks, pre_m, k2, sh, st); break;
+      default: ksum_lu_go<4>(n, N, nblk, nb, nq, ent, rowptr, Pw, Glso + o, nks, Mt, kw, fp, kchunks, pre_m, k2, sh, st); break;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------

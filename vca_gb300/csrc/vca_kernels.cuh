@@ -128,8 +128,9 @@ struct GfLayout {
   const int* elem_chain;  // chain ids
   ChainStore cs;          // the chains' tridiagonals
 };
-// raw element sums at nz points z (complex): G[z*nelem + e]
-void launch_gf_eval(const GfLayout& g, int nz, const double2* z, double2* G, cudaStream_t st);
+// raw element sums at nz points z (complex): G[z*nelem + e]; val: nch*nz
+// values of the store's nch chains
+void launch_gf_eval(const GfLayout& g, int nch, int nz, const double2* z, double2* val, double2* G, cudaStream_t st);
 // the same raw sums from pole tables (a GFmatrix read from a restart file):
 // G[z*nelem + e] = sum over ptr[e] <= x < ptr[e+1] of weights[x] / (z - poles[x])
 void launch_gf_eval_poles(int nelem, const int64_t* ptr, const double2* poles, const double2* weights, int nz,
@@ -159,6 +160,14 @@ struct KsumInverse {
 void launch_omega_ksum2(int nw, int N, int nblk, int nb, const double2* P, const double2* Glso, int64_t Nk,
                         const double2* Hk, const double* kw, const int* rowptr, const int* cols, double* fpart,
                         double* fpart_im, int kchunks, bool pre_m, const KsumInverse& ki, cudaStream_t st);
+// The T=0 integrand (real part) by whole determinants per thread, where
+// ksum_lu_ok: the pattern as nq entries by rows (rowptr), il = their lso element
+// index, ent = row | col << 8 within the block; M as Hk above, Mt: nq*nks scratch
+bool ksum_lu_ok(int N, int nblk, int nb, int nq, bool pre_m);
+void launch_ksum_lu(int nw, int N, int nblk, int nb, int nq, const int* il, const int* ent, const int* rowptr,
+                    const double2* P, const double2* Glso, int64_t nks, const double2* M, double2* Mt,
+                    const double* kw, double* fpart, int kchunks, bool pre_m, const KsumInverse& ki,
+                    cudaStream_t st);
 // G'^-1 and ln|det G'| of each diagonal block (nblk blocks of nb <= 32) of n lso matrices
 void launch_ginv_blocks(int n, int N, int nblk, int nb, const double2* Glso, double2* Ginv, double* ldG,
                         cudaStream_t st);
