@@ -129,6 +129,9 @@ struct Ctx {
     unsigned* hop = nullptr;
     unsigned* rhop = nullptr;
     int* pinv = nullptr;
+    unsigned* p16 = nullptr;       // packed pairs (FxView::up_p16), large spaces with one class
+    unsigned short* n16 = nullptr;
+    int w16 = 0;
     int *cnt = nullptr, *npos = nullptr, *word = nullptr;
     i64* e1 = nullptr;
   };
@@ -306,6 +309,9 @@ FxView fx_view_pair(int sa, int na, int sb, int nb) {
   const Ctx::PermTabs& pt = g->fx_ptab[sa][na];
   f.up_phop = pt.hop;
   f.up_rhop = pt.rhop;
+  f.up_p16 = pt.p16;
+  f.up_n16 = pt.n16;
+  f.w16 = pt.w16;
   f.up_pinv = pt.pinv;
   f.rows_permuted = 0;
   f.up_pcnt = pt.cnt;
@@ -590,6 +596,13 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
             fx_rhop_parity_order(S.dim, S.width, pc.data(), pn.data(), rh.data());
             CUCHK(cudaMemcpyAsync(pt.rhop, rh.data(), sizeof(unsigned) * rh.size(), cudaMemcpyHostToDevice, g->st));
             CUCHK(cudaStreamSynchronize(g->st));
+          }
+          // packed for the column product of spaces that the resident runs leave to it
+          if (fb.K == 1 && S.dim >= 128 && S.dim <= 1023 && S.width > 0 && S.width <= 500) {
+            pt.w16 = fx_p16_width(S.width);
+            RCHK(g->ham.alloc(&pt.p16, 2 * (size_t)pt.w16 * S.dim));
+            RCHK(g->ham.alloc(&pt.n16, S.dim));
+            launch_fx_pack16(S.dim, S.width, pt.cnt, pt.npos, pt.rhop, pt.p16, pt.n16, g->st);
           }
           if (S.dim > 0 && fx_pair_fits(S.dim) && (int64_t)S.dim * partner >= FX1_MIN_DIM) {
             std::vector<int> cnt(S.dim);

@@ -1142,6 +1142,29 @@ void launch_fx_perm_tables(int dim, int width, const int* perm, const int* pinv,
                                                       rhop, pcnt, pnpos, pword, pe1);
 }
 
+__global__ void k_fx_pack16(int dim, int width, const int* cnt, const int* npos, const unsigned* rhop, unsigned* p16,
+                            unsigned short* n16) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= dim) return;
+  const int w16 = fx_p16_width(width), n = cnt[i], np = npos[i];
+  for (int sg = 0; sg < 2; sg++) {
+    const int h0 = sg ? np : 0, h1 = sg ? n : np;
+    for (int w = 0; w < w16; w++) {
+      const int h = h0 + 2 * w;
+      const unsigned a = h < h1 ? rhop[(int64_t)h * dim + i] & 0xFFFFu : (unsigned)dim;
+      const unsigned b = h + 1 < h1 ? rhop[(int64_t)(h + 1) * dim + i] & 0xFFFFu : (unsigned)dim;
+      p16[(int64_t)(sg * w16 + w) * dim + i] = 64u * a | (64u * b) << 16;
+    }
+  }
+  n16[i] = (unsigned short)((np + 1) / 2 | ((n - np + 1) / 2) << 8);
+}
+void launch_fx_pack16(int dim, int width, const int* cnt, const int* npos, const unsigned* rhop, unsigned* p16,
+                      unsigned short* n16, cudaStream_t st) {
+  if (dim == 0) return;
+  count_launch_external();
+  k_fx_pack16<<<(dim + 127) / 128, 128, 0, st>>>(dim, width, cnt, npos, rhop, p16, n16);
+}
+
 // accumulate one hop's source row into the class accumulators; the class and
 // sign are warp-uniform, so the branches do not diverge.  xr points at the
 // source row's first column within slab 0; coff[q] adds lane column q's slab
@@ -1553,6 +1576,35 @@ __device__ __forceinline__ void fxb_start(uint32_t bar, uint32_t dst, const void
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
+// the CTA's alpha partials: column sums over its rows to row idw of `apart`
+__device__ __forceinline__ void fxr_store_alpha(i128 ad0, i128 ad1, int u, int lane, int warp, int nwarp, int c0, int m,
+                                                int idw, i64* apart) {
+  constexpr int W = FX_SLAB;
+  __shared__ i128 red[32][W];
+  i128 adv[2] = {ad0, ad1};
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    u64 lo = (u64)adv[j];
+    i64 hi = (i64)(adv[j] >> 64);
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) {  // lanes holding the same columns
+      const u64 lo2 = __shfl_xor_sync(0xffffffffu, lo, off);
+      const i64 hi2 = __shfl_xor_sync(0xffffffffu, hi, off);
+      const u64 sl = lo + lo2;
+      hi = hi + hi2 + (sl < lo ? 1 : 0);
+      lo = sl;
+    }
+    if (lane < 4) red[warp][2 * u + j] = ((i128)hi << 64) | (i128)lo;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < W && c0 + (int)threadIdx.x < m) {
+    i128 sum = 0;
+    for (int w = 0; w < nwarp; w++) sum += red[w][threadIdx.x];
+    const int64_t o2 = 2 * ((int64_t)idw * m + c0 + threadIdx.x);
+    apart[o2] = (i64)(u64)sum;
+    apart[o2 + 1] = (i64)(sum >> 64);
+  }
+}
 template <int K, bool SH63, bool APART>
 __global__ void __launch_bounds__(FXR_THREADS, 4) k_hxv_fx_r(SectorView sv, FxView fv, int m,
                                                               const i64* __restrict__ X, i64* __restrict__ Y,
@@ -1678,37 +1730,136 @@ __global__ void __launch_bounds__(FXR_THREADS, 4) k_hxv_fx_r(SectorView sv, FxVi
       }
     }
   }
-  if (APART) {
-    __shared__ i128 red[FXR_THREADS / 32][W];
-    i128 adv[2] = {ad0, ad1};
+  if (APART) fxr_store_alpha(ad0, ad1, u, lane, warp, nwarp, c0, m, idw, apart);
+}
+
+// The same product for one amplitude class (K = 1) with the up hops packed two
+// to a word (FxView::up_p16).  In the form above every hop waits for its table
+// word, and the 38 KB table of the 4x3 chain sectors misses the 20 KB of L1
+// that four CTAs' blocks leave; here a word brings two gathers, both rows of a
+// lane loop together (past a row's end a word points at the zero row), so a
+// pass has four independent gathers in flight, and the words in use are 17 KB.
+// Bound by issue (62 %) and the latency of table words and neighbour rows; of
+// its time the up hops take 36 %, the down hops 26 %, the 128-bit products 16 %.
+// 408 columns of the 4x3 sector (7,6): 3.74 -> 3.09 ms, 1.55 TB/s of algorithmic
+// traffic (256 threads 3.16, 320 in three CTAs 3.11, 512 in two 3.28; hop
+// loops unrolled twice 3.25; the products written out in 32-bit words 3.32).
+#define FXP_THREADS 288  // 9 warps: the fourth CTA still fits the register file
+#define FXP_BLOCKS 4
+template <bool SH63, bool APART>
+__global__ void __launch_bounds__(FXP_THREADS, FXP_BLOCKS) k_hxv_fx_p(SectorView sv, FxView fv, int m,
+                                                              const i64* __restrict__ X, i64* __restrict__ Y,
+                                                              i64* __restrict__ apart) {
+  extern __shared__ __align__(16) unsigned char fxp_smem[];
+  constexpr int W = FX_SLAB;
+  const int DU = sv.dimup, DD = sv.dimdw;
+  const int64_t D = (int64_t)DU * DD;
+  longlong2* xs2 = (longlong2*)fxp_smem;  // [DU + 1][4] own block, position order, and a zero row
+  unsigned long long* sbar = (unsigned long long*)(xs2 + (size_t)(DU + 1) * 4);
+  int* doff = (int*)(sbar + 2);  // down hops: offsets in 16-byte units
+  const int cs = blockIdx.x / DD;
+  const int idw = blockIdx.x - cs * DD;
+  const int c0 = cs * W;
+  const int64_t rowbase = (int64_t)idw * DU;
+  const longlong2* own = (const longlong2*)X + (int64_t)cs * D * (W / 2) + rowbase * 4;
+  longlong2* yown = (longlong2*)Y + (int64_t)cs * D * (W / 2) + rowbase * 4;
+  const int nd = sv.dw_cnt[idw];
+  const int ndp = fv.dw_npos[idw];
+  __shared__ int stage_ok;  // as k_hxv_fx_r
+  const uint32_t bar_s = (uint32_t)__cvta_generic_to_shared(sbar);
+  if (threadIdx.x == 0)
+    fxb_start(bar_s, (uint32_t)__cvta_generic_to_shared(xs2), own, (uint32_t)DU * 64u);
+  for (int h = threadIdx.x; h < nd; h += blockDim.x)
+    doff[h] = ((int)(fv.dw_hop[idw + h * DD] & 0xFFFFFFu) - idw) * DU * 4;
+  if (threadIdx.x < 4) xs2[DU * 4 + threadIdx.x] = make_longlong2(0, 0);
+  if (threadIdx.x == 0) {
+    const bool ok = fxb_wait_bounded(bar_s, 0);
+    if (!ok) {
+      atomicAdd(&g_fx_wait_fail, 1);
+      fxb_wait_bounded(bar_s, 0);
+    }
+    stage_ok = ok ? 1 : 0;
+  }
+  __syncthreads();
+  if (!stage_ok) return;
+  for (int it = 0; it < (1 << 16) && !fxb_try_wait(bar_s, 0); it++) {
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int u = lane & 3, rsub = lane >> 2;
+  const i64 e1d = fv.dw_e1[idw];
+  const unsigned wdw = (unsigned)sv.dw_words[idw];
+  const unsigned* __restrict__ tab = fv.up_p16;
+  const int w16 = fv.w16;
+  const longlong2* xu = xs2 + u;
+  const unsigned ub = 16u * (unsigned)u;  // the lane's unit within a 64-byte row
+#define FXP_AT(off) (*(const longlong2*)(fxp_smem + (off)))
+  i128 ad0 = 0, ad1 = 0;
+  for (int pb = warp * 16; pb < DU; pb += nwarp * 16) {
+    const int pr0 = pb + rsub, pr1 = pb + 8 + rsub;
+    const bool ok0 = pr0 < DU, ok1 = pr1 < DU;
+    const int q0 = ok0 ? pr0 : 0, q1 = ok1 ? pr1 : 0;  // rows past the end repeat row 0 and are not stored
+    u64 S[2][2] = {{0, 0}, {0, 0}};
+    const longlong2* a0 = own + q0 * 4 + u;
+    const longlong2* a1 = own + q1 * 4 + u;
+    int h = 0;
+#pragma unroll 2
+    for (; h < ndp; h++) {
+      const int o = doff[h];
+      const longlong2 v0 = __ldcg(a0 + o), v1 = __ldcg(a1 + o);
+      S[0][0] += (u64)v0.x; S[0][1] += (u64)v0.y; S[1][0] += (u64)v1.x; S[1][1] += (u64)v1.y;
+    }
+#pragma unroll 2
+    for (; h < nd; h++) {
+      const int o = doff[h];
+      const longlong2 v0 = __ldcg(a0 + o), v1 = __ldcg(a1 + o);
+      S[0][0] -= (u64)v0.x; S[0][1] -= (u64)v0.y; S[1][0] -= (u64)v1.x; S[1][1] -= (u64)v1.y;
+    }
+    const unsigned n0 = fv.up_n16[q0], n1 = fv.up_n16[q1];
+    const int np = max(n0 & 255u, n1 & 255u), nn = max(n0 >> 8, n1 >> 8);
+    const unsigned* t0 = tab + q0;
+    const unsigned* t1 = tab + q1;
+#pragma unroll 1
+    for (int k = 0; k < np; k++) {
+      const unsigned w0 = t0[k * DU], w1 = t1[k * DU];
+      const longlong2 a = FXP_AT((w0 & 0xFFFFu) | ub), b = FXP_AT((w0 >> 16) | ub);
+      const longlong2 c = FXP_AT((w1 & 0xFFFFu) | ub), d = FXP_AT((w1 >> 16) | ub);
+      S[0][0] += (u64)a.x + (u64)b.x; S[0][1] += (u64)a.y + (u64)b.y;
+      S[1][0] += (u64)c.x + (u64)d.x; S[1][1] += (u64)c.y + (u64)d.y;
+    }
+    t0 += w16 * DU;
+    t1 += w16 * DU;
+#pragma unroll 1
+    for (int k = 0; k < nn; k++) {
+      const unsigned w0 = t0[k * DU], w1 = t1[k * DU];
+      const longlong2 a = FXP_AT((w0 & 0xFFFFu) | ub), b = FXP_AT((w0 >> 16) | ub);
+      const longlong2 c = FXP_AT((w1 & 0xFFFFu) | ub), d = FXP_AT((w1 >> 16) | ub);
+      S[0][0] -= (u64)a.x + (u64)b.x; S[0][1] -= (u64)a.y + (u64)b.y;
+      S[1][0] -= (u64)c.x + (u64)d.x; S[1][1] -= (u64)c.y + (u64)d.y;
+    }
 #pragma unroll
     for (int j = 0; j < 2; j++) {
-      u64 lo = (u64)adv[j];
-      i64 hi = (i64)(adv[j] >> 64);
-#pragma unroll
-      for (int off = 4; off < 32; off <<= 1) {  // lanes holding the same columns
-        const u64 lo2 = __shfl_xor_sync(0xffffffffu, lo, off);
-        const i64 hi2 = __shfl_xor_sync(0xffffffffu, hi, off);
-        const u64 sl = lo + lo2;
-        hi = hi + hi2 + (sl < lo ? 1 : 0);
-        lo = sl;
+      if (!(j ? ok1 : ok0)) continue;
+      const int p = j ? pr1 : pr0;
+      const longlong2 x = xu[p * 4];
+      const i64 dfx = fv.up_pe1[p] + e1d + mixed_fx(fv, (unsigned)fv.up_pword[p], wdw);
+      const i128 r0 = (i128)dfx * x.x + (i128)fv.afx[0] * (i64)S[j][0];
+      const i128 r1 = (i128)dfx * x.y + (i128)fv.afx[0] * (i64)S[j][1];
+      const i64 y0 = SH63 ? rshift_round63(r0, fv.shift) : rshift_round(r0, fv.shift);
+      const i64 y1 = SH63 ? rshift_round63(r1, fv.shift) : rshift_round(r1, fv.shift);
+      __stcs(yown + p * 4 + u, make_longlong2(y0, y1));
+      if (APART) {
+        if (c0 + 2 * u < m) ad0 += (i128)x.x * y0;
+        if (c0 + 2 * u + 1 < m) ad1 += (i128)x.y * y1;
       }
-      if (lane < 4) red[warp][2 * u + j] = ((i128)hi << 64) | (i128)lo;
-    }
-    __syncthreads();
-    if ((int)threadIdx.x < W && c0 + (int)threadIdx.x < m) {
-      i128 sum = 0;
-      for (int w = 0; w < nwarp; w++) sum += red[w][threadIdx.x];
-      const int64_t o2 = 2 * ((int64_t)idw * m + c0 + threadIdx.x);
-      apart[o2] = (i64)(u64)sum;
-      apart[o2 + 1] = (i64)(sum >> 64);
     }
   }
+#undef FXP_AT
+  if (APART) fxr_store_alpha(ad0, ad1, u, lane, warp, nwarp, c0, m, idw, apart);
 }
 
 #define FXR_SMEM_MAX (200 * 1024)
 static size_t hxv_fx_r_smem(const SectorView& sv) {
-  return (size_t)sv.dimup * FX_SLAB * sizeof(i64) + 16 + (size_t)sv.wdw * 5 + 16;
+  return (size_t)(sv.dimup + 1) * FX_SLAB * sizeof(i64) + 16 + (size_t)sv.wdw * 5 + 16;
 }
 
 int fx_take_wait_failures() {
@@ -1742,9 +1893,29 @@ static void launch_hxv_fx_r_t(const SectorView& sv, const FxView& fv, int m, con
   count_launch_external();
   k_hxv_fx_r<K, SH63, APART><<<sv.dimdw * ns, FXR_THREADS, hxv_fx_r_smem(sv), st>>>(sv, fv, m, X, Y, apart);
 }
+template <bool SH63, bool APART>
+static void launch_hxv_fx_p_t(const SectorView& sv, const FxView& fv, int m, const i64* X, i64* Y, i64* apart,
+                              cudaStream_t st) {
+  static bool attr_set = false;  // per instantiation, process-wide (every device is sm_103a)
+  if (!attr_set) {
+    cudaFuncSetAttribute(k_hxv_fx_p<SH63, APART>, cudaFuncAttributeMaxDynamicSharedMemorySize, FXR_SMEM_MAX);
+    attr_set = true;
+  }
+  const int ns = (m + FX_SLAB - 1) / FX_SLAB;
+  count_launch_external();
+  k_hxv_fx_p<SH63, APART><<<sv.dimdw * ns, FXP_THREADS, hxv_fx_r_smem(sv), st>>>(sv, fv, m, X, Y, apart);
+}
 template <int K>
 static void launch_hxv_fx_r_k(const SectorView& sv, const FxView& fv, int m, const i64* X, i64* Y, i64* apart,
                               cudaStream_t st) {
+  if (K == 1 && fv.up_p16) {
+    const bool s63 = fv.shift >= 1 && fv.shift <= 63;
+    if (s63 && apart) launch_hxv_fx_p_t<true, true>(sv, fv, m, X, Y, apart, st);
+    else if (s63) launch_hxv_fx_p_t<true, false>(sv, fv, m, X, Y, apart, st);
+    else if (apart) launch_hxv_fx_p_t<false, true>(sv, fv, m, X, Y, apart, st);
+    else launch_hxv_fx_p_t<false, false>(sv, fv, m, X, Y, apart, st);
+    return;
+  }
   const bool sh63 = fv.shift >= 1 && fv.shift <= 63;
   if (sh63 && apart) launch_hxv_fx_r_t<K, true, true>(sv, fv, m, X, Y, apart, st);
   else if (sh63) launch_hxv_fx_r_t<K, true, false>(sv, fv, m, X, Y, apart, st);

@@ -53,6 +53,14 @@ struct FxView {
   const unsigned* up_rhop;     // the same hops with the source as its position in up_perm
   const int* up_pinv;          // position of each up configuration in up_perm
   int rows_permuted;           // 1: the batch's fast-index rows are in up_perm order
+  // the same hops for one amplitude class, two a word as 16-bit byte offsets of
+  // 64-byte rows, the positive hops in up_p16[0 .. w16) and the negative ones
+  // in up_p16[w16 .. 2 w16) (k-major); an unused half points at the zero row
+  // (position dim, so dim <= 1023);
+  // up_n16: words used, positive | negative << 8.  nullptr: not built
+  const unsigned* up_p16;
+  const unsigned short* up_n16;
+  int w16;
   const int* up_pcnt;
   const int* up_pnpos;
   const int* up_pword;
@@ -89,6 +97,11 @@ __host__ __device__ __forceinline__ int64_t fx_off(int64_t D, int W, int64_t i, 
   return ((int64_t)(c / W) * D + i) * W + c % W;
 }
 
+// the packed table of FxView::up_p16 from rhop (cnt, npos per row), w16 =
+// fx_p16_width(width) words per sign
+__host__ __device__ inline int fx_p16_width(int width) { return (width + 1) / 2; }
+void launch_fx_pack16(int dim, int width, const int* cnt, const int* npos, const unsigned* rhop, unsigned* p16,
+                      unsigned short* n16, cudaStream_t st);
 // up-spin tables in the order of perm (see FxView::up_phop)
 void launch_fx_perm_tables(int dim, int width, const int* perm, const int* pinv, const unsigned* hop,
                            const int* cnt, const int* npos, const int* words, const i64* e1, unsigned* phop,
