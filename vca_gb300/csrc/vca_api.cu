@@ -55,14 +55,37 @@ std::string g_err;
     if (r_ != VCA_OK) return r_; \
   } while (0)
 
+// The context's stream-ordered memory pool, made by vca_gpu_init and destroyed
+// by vca_gpu_finalize.  A solve makes hundreds of small allocations; from the
+// driver each costs 3-4 us and as much again, with a device synchronisation,
+// when it is freed (1.4 of the 3.0 ms of a 2x2 solve).  The pool keeps at most
+// POOL_KEEP bytes between calls and returns what is above that to the device
+// at the next synchronisation.
+#define POOL_KEEP ((uint64_t)256 << 20)
+cudaMemPool_t g_pool = nullptr;
+cudaStream_t g_pool_stream = nullptr;  // the context's stream
+
+// free device memory as a budget sees it: what the pool holds unused and
+// above its bound is given back first
+cudaError_t free_memory(size_t* freeb, size_t* totb) {
+  if (g_pool) {
+    const cudaError_t e = cudaStreamSynchronize(g_pool_stream);
+    if (e != cudaSuccess) return e;
+    cudaMemPoolTrimTo(g_pool, (size_t)POOL_KEEP);
+  }
+  return cudaMemGetInfo(freeb, totb);
+}
+
 // Device allocations owned by one stage of the context.
 struct Arena {
   std::vector<void*> ptrs;
+  cudaStream_t st = nullptr;  // the stream they are used on; nullptr: the context's
   template <class T>
   int alloc(T** p, size_t n) {
     *p = nullptr;
     if (n == 0) n = 1;
-    cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+    cudaError_t e = g_pool ? cudaMallocFromPoolAsync((void**)p, n * sizeof(T), g_pool, st ? st : g_pool_stream)
+                           : cudaMalloc((void**)p, n * sizeof(T));
     if (e != cudaSuccess) {
       *p = nullptr;
       g_err = std::string("cudaMalloc of ") + std::to_string(n * sizeof(T)) + " bytes failed: " +
@@ -74,7 +97,10 @@ struct Arena {
     return VCA_OK;
   }
   void release() {
-    for (void* p : ptrs) cudaFree(p);
+    for (void* p : ptrs) {
+      if (g_pool) cudaFreeAsync(p, st ? st : g_pool_stream);
+      else cudaFree(p);
+    }
     ptrs.clear();
   }
 };
@@ -727,13 +753,14 @@ int lanczos_step_fx(const SectorView& sv, const FxView& fv, const ColBatch& cb, 
 }
 
 int alloc_batch(Arena& ar, int64_t rows, int m, bool cplx, int nch, int ldab, BatchBufs& bb) {
+  const cudaStream_t st = ar.st ? ar.st : g->st;  // where the batch runs
   const size_t es = cplx ? sizeof(double2) : sizeof(double);
   // fixed-point batches are slab-major with zero pad columns
   const int mc = g->fx ? fx_cols_alloc(m) : m;
   for (int q = 0; q < 3; q++) {
     char* p;
     RCHK(ar.alloc(&p, (size_t)rows * mc * es));
-    if (mc > m) CUCHK(cudaMemsetAsync(p, 0, (size_t)rows * mc * es, g->st));
+    if (mc > m) CUCHK(cudaMemsetAsync(p, 0, (size_t)rows * mc * es, st));
     bb.b[q] = p;
   }
   bb.nblk = (int)std::min<int64_t>(std::max<int64_t>(1, rows / 256), 608);
@@ -752,9 +779,9 @@ int alloc_batch(Arena& ar, int64_t rows, int m, bool cplx, int nch, int ldab, Ba
   RCHK(ar.alloc(&bb.Bt, (size_t)nch * ldab));
   RCHK(ar.alloc(&bb.meta, nch));
   RCHK(ar.alloc(&bb.col2ch, m));
-  CUCHK(cudaMemsetAsync(bb.A, 0, sizeof(double) * nch * ldab, g->st));
-  CUCHK(cudaMemsetAsync(bb.Bt, 0, sizeof(double) * nch * ldab, g->st));
-  CUCHK(cudaMemsetAsync(bb.bnow, 0, sizeof(double) * nch, g->st));
+  CUCHK(cudaMemsetAsync(bb.A, 0, sizeof(double) * nch * ldab, st));
+  CUCHK(cudaMemsetAsync(bb.Bt, 0, sizeof(double) * nch * ldab, st));
+  CUCHK(cudaMemsetAsync(bb.bnow, 0, sizeof(double) * nch, st));
   return VCA_OK;
 }
 
@@ -1809,7 +1836,7 @@ int chain_groups(const ChainList& list, int npar, std::vector<ChainGroup>& out) 
   const bool cplx = !g->real_model;
   const size_t es = cplx ? sizeof(double2) : sizeof(double);
   size_t freeb = 0, totb = 0;
-  CUCHK(cudaMemGetInfo(&freeb, &totb));
+  CUCHK(free_memory(&freeb, &totb));
   const size_t budget = (size_t)(0.5 * (double)freeb / std::max(1, npar));
   int64_t maxcols = (int64_t)(budget / (3 * (size_t)D * es + 1));
   if (g->fx && maxcols > FX_SLAB) maxcols = maxcols / FX_SLAB * FX_SLAB;  // room for the pad columns
@@ -1846,6 +1873,7 @@ int chain_group_prepare(ChainGroup& G) {
   const int nup = sec_nup(S.sector);
   const bool cplx = !g->real_model;
   const int m = G.m, nch = G.nch;
+  G.ar.st = G.st;
   int rc = alloc_batch(G.ar, G.D, m, cplx, nch, g->ld, G.bb);
   BatchBufs& bb = G.bb;
   // fixed-point batches hold the smaller spin block first (see view_pair),
@@ -3344,7 +3372,7 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
   while (p0 < B) {
     // ---- 1. tables of a wave of points ---------------------------------------
     size_t freeb = 0, totb = 0;
-    if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess) { restore(); VFAIL(VCA_ERR_CUDA, "cudaMemGetInfo failed"); }
+    if (free_memory(&freeb, &totb) != cudaSuccess) { restore(); VFAIL(VCA_ERR_CUDA, "cudaMemGetInfo failed"); }
     const size_t per_point = 3 * (size_t)sumD * sizeof(double2) + ((size_t)8 << 20);
     const int P = (int)std::max<int64_t>(1, std::min<int64_t>(B - p0, (int64_t)(0.35 * (double)freeb / per_point)));
     const int p1 = p0 + P;
@@ -3627,7 +3655,7 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
         }
       }
       size_t fb = 0;
-      cudaMemGetInfo(&fb, &totb);
+      free_memory(&fb, &totb);
       const size_t gbudget = (size_t)(0.3 * (double)fb);
       size_t t0i = 0;
       while (t0i < trefs.size()) {
@@ -3848,6 +3876,12 @@ int vca_gpu_finalize(void) {
   g->ham.release();
   g->basis.release();
   g->rs.drop();
+  if (g_pool) {  // every allocation is back
+    cudaStreamSynchronize(g_pool_stream);
+    cudaMemPoolDestroy(g_pool);
+    g_pool = nullptr;
+    g_pool_stream = nullptr;
+  }
   if (g->st) cudaStreamDestroy(g->st);
   if (g->st2) cudaStreamDestroy(g->st2);
   delete g;
@@ -3910,6 +3944,21 @@ int vca_gpu_init(const vca_config* cfg, const double* bath_h, const double* bath
   // a blocking stream: the synchronous getters on the legacy stream order after it
   CUCHK(cudaStreamCreate(&g->st));
   CUCHK(cudaStreamCreate(&g->st2));
+  {
+    int dev = 0, pools = 0;
+    CUCHK(cudaGetDevice(&dev));
+    CUCHK(cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, dev));
+    if (pools) {
+      cudaMemPoolProps pp{};
+      pp.allocType = cudaMemAllocationTypePinned;
+      pp.location.type = cudaMemLocationTypeDevice;
+      pp.location.id = dev;
+      CUCHK(cudaMemPoolCreate(&g_pool, &pp));
+      uint64_t keep = POOL_KEEP;
+      CUCHK(cudaMemPoolSetAttribute(g_pool, cudaMemPoolAttrReleaseThreshold, &keep));
+      g_pool_stream = g->st;
+    }
+  }
   set_binomials(Ns, g->st);
   g->dimn.resize(Ns + 1);
   g->words.resize(Ns + 1);
