@@ -522,7 +522,8 @@ int vca_gpu_set_autotune(int32_t on);
  * reads its up hops in an order that pairs the two rows of each quarter
  * warp with sources of opposite parity, so their 16-byte shared-memory
  * reads fall in different banks (on = 1, default); on = 0 keeps the plain
- * sign-sorted order.  Takes effect when the next Hamiltonian's tables are
+ * sign-sorted order.  Applies to up spaces of 128 configurations and more (the
+ * chains of smaller ones run in one launch), when the next Hamiltonian's tables are
  * built; results are bit-identical either way.  No counterpart in the
  * reference. */
 int vca_gpu_set_hop_pairing(int32_t on);

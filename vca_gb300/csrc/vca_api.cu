@@ -487,15 +487,22 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
       g->host_eps_abs.push_back(em * g->Ns + std::fabs(ep.upar) * c.Nlat * c.Norb * c.Norb);
     }
     g->sp[set].assign(g->Ns + 1, SpinSpace());
+    // every filling's counts, then their widths in one read
+    int widths[VCA_MAX_NS + 1];
+    CUCHK(cudaMemsetAsync(g->d_iscratch, 0, sizeof(int) * (g->Ns + 1), g->st));
     for (int n = 0; n <= g->Ns; n++) {
       SpinSpace& S = g->sp[set][n];
       S.n = n;
       S.dim = g->dimn[n];
       S.words = g->words[n];
       RCHK(g->ham.alloc(&S.cnt, S.dim));
-      S.width = launch_hop_count(g->Ns, n, S.dim, S.words, g->d_pairs[set], (int)pairs.size(), S.cnt,
-                                 g->d_iscratch, g->st);
-      CUCHK(cudaGetLastError());
+      launch_hop_count(S.dim, S.words, g->d_pairs[set], (int)pairs.size(), S.cnt, g->d_iscratch + n, g->st);
+    }
+    CUCHK(cudaMemcpyAsync(widths, g->d_iscratch, sizeof(int) * (g->Ns + 1), cudaMemcpyDeviceToHost, g->st));
+    CUCHK(cudaStreamSynchronize(g->st));
+    for (int n = 0; n <= g->Ns; n++) {
+      SpinSpace& S = g->sp[set][n];
+      S.width = widths[n];
       RCHK(g->ham.alloc(&S.src, (size_t)S.width * S.dim));
       RCHK(g->ham.alloc(&S.amp, (size_t)S.width * S.dim));
       RCHK(g->ham.alloc(&S.e1, S.dim));
@@ -583,15 +590,20 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
           launch_fx_pack(S.dim, S.width, S.src, S.amp, d_cls, fb.K, g->fx_hop[set][n], g->st);
           RCHK(g->ham.alloc(&g->fx_npos[set][n], S.dim));
           launch_fx_sign_sort(S.dim, S.width, S.cnt, g->fx_hop[set][n], g->fx_npos[set][n], g->st);
-          {  // rows by decreasing hop count (stable), for warps of equal loop length
+          RCHK(g->ham.alloc(&g->fx_perm[set][n], S.dim));
+          RCHK(g->ham.alloc(&g->fx_ptab[set][n].pinv, S.dim));
+          // rows by decreasing hop count (stable), for warps of equal loop length; the
+          // device's dim^2 comparisons against a sort on the host and its copies
+          // (100 us a space): 40 us at the 12,870 rows of the 4x4 cluster
+          if (S.dim <= 1 << 14) {
+            launch_hop_order(S.dim, S.cnt, g->fx_perm[set][n], g->fx_ptab[set][n].pinv, g->st);
+          } else {
             std::vector<int> cnt(S.dim), perm(S.dim);
             if (S.dim) CUCHK(cudaMemcpy(cnt.data(), S.cnt, sizeof(int) * S.dim, cudaMemcpyDeviceToHost));
             for (int r = 0; r < S.dim; r++) perm[r] = r;
             std::stable_sort(perm.begin(), perm.end(), [&](int x, int y) { return cnt[x] > cnt[y]; });
             std::vector<int> pinv(S.dim);
             for (int r = 0; r < S.dim; r++) pinv[perm[r]] = r;
-            RCHK(g->ham.alloc(&g->fx_perm[set][n], S.dim));
-            RCHK(g->ham.alloc(&g->fx_ptab[set][n].pinv, S.dim));
             if (S.dim) {
               CUCHK(cudaMemcpy(g->fx_perm[set][n], perm.data(), sizeof(int) * S.dim, cudaMemcpyHostToDevice));
               CUCHK(cudaMemcpy(g->fx_ptab[set][n].pinv, pinv.data(), sizeof(int) * S.dim, cudaMemcpyHostToDevice));
@@ -611,8 +623,9 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
           launch_fx_perm_tables(S.dim, S.width, g->fx_perm[set][n], pt.pinv, g->fx_hop[set][n], S.cnt,
                                 g->fx_npos[set][n], S.words, g->fx_e1[set][n], pt.hop, pt.rhop, pt.cnt, pt.npos,
                                 pt.word, pt.e1, g->st);
-          if (S.dim > 1 && (size_t)S.dim * FX_SLAB * sizeof(i64) <= 200 * 1024 && g->rhop_order) {
+          if (S.dim >= 128 && (size_t)S.dim * FX_SLAB * sizeof(i64) <= 200 * 1024 && g->rhop_order) {
             // the position-ordered kernel's up block fits: pair its rows' hop parities
+            // (smaller spaces' chains run resident, vca_resident.cuh)
             std::vector<int> pc(S.dim), pn(S.dim);
             std::vector<unsigned> rh((size_t)S.width * S.dim);
             CUCHK(cudaMemcpyAsync(pc.data(), pt.cnt, sizeof(int) * S.dim, cudaMemcpyDeviceToHost, g->st));
@@ -3967,7 +3980,7 @@ int vca_gpu_init(const vca_config* cfg, const double* bath_h, const double* bath
     RCHK(g->basis.alloc(&g->words[n], g->dimn[n]));
     launch_build_words(Ns, n, g->dimn[n], g->words[n], g->st);
   }
-  RCHK(g->basis.alloc(&g->d_iscratch, 16));
+  RCHK(g->basis.alloc(&g->d_iscratch, VCA_MAX_NS + 1));
   CUCHK(cudaGetLastError());
   CUCHK(cudaStreamSynchronize(g->st));
   return VCA_OK;

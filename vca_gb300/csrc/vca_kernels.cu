@@ -100,17 +100,35 @@ __global__ void k_hop_count(int dim, const int* words, const HopPair* pairs, int
   }
   atomicMax(gmax, local_max);
 }
-int launch_hop_count(int Ns, int n, int dim, const int* words, const HopPair* d_pairs, int npairs,
-                     int* cnt, int* d_scratch_max, cudaStream_t st) {
+void launch_hop_count(int dim, const int* words, const HopPair* d_pairs, int npairs, int* cnt, int* d_max,
+                      cudaStream_t st) {
   COUNT_LAUNCH();
-  (void)Ns;
-  (void)n;
-  cudaMemsetAsync(d_scratch_max, 0, sizeof(int), st);
-  k_hop_count<<<nblocks(dim, 256), 256, 0, st>>>(dim, words, d_pairs, npairs, cnt, d_scratch_max);
-  int h = 0;
-  cudaMemcpyAsync(&h, d_scratch_max, sizeof(int), cudaMemcpyDeviceToHost, st);
-  cudaStreamSynchronize(st);
-  return h;
+  k_hop_count<<<nblocks(dim, 256), 256, 0, st>>>(dim, words, d_pairs, npairs, cnt, d_max);
+}
+
+// Rows by decreasing hop count, stable: each row's place is the number of
+// rows before it, counted in chunks of rows staged in shared memory.
+__global__ void k_hop_order(int dim, const int* cnt, int* perm, int* pinv) {
+  __shared__ int c[1024];
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int mine = r < dim ? cnt[r] : 0;
+  int q = 0;
+  for (int i0 = 0; i0 < dim; i0 += 1024) {
+    const int n = min(1024, dim - i0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) c[i] = cnt[i0 + i];
+    __syncthreads();
+    for (int i = 0; i < n; i++) q += c[i] > mine || (c[i] == mine && i0 + i < r);
+  }
+  if (r < dim) {
+    perm[q] = r;
+    pinv[r] = q;
+  }
+}
+void launch_hop_order(int dim, const int* cnt, int* perm, int* pinv, cudaStream_t st) {
+  if (dim <= 0) return;
+  COUNT_LAUNCH();
+  k_hop_order<<<(dim + 127) / 128, 128, 0, st>>>(dim, cnt, perm, pinv);
 }
 
 __global__ void k_hop_fill(int dim, int width, const int* words, const HopPair* pairs, int npairs,

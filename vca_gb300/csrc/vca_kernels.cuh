@@ -23,9 +23,12 @@ struct E1Params {    // one-body + same-spin diagonal energy of a spin word
   int norb;
   unsigned int omask[VCA_MAX_NORB];
 };
-// count hops per target word and return the ELL width (max count)
-int launch_hop_count(int Ns, int n, int dim, const int* words, const HopPair* d_pairs, int npairs,
-                     int* cnt, int* d_scratch_max, cudaStream_t st);
+// hops per target word; *d_max gains the ELL width (most hops of a word)
+void launch_hop_count(int dim, const int* words, const HopPair* d_pairs, int npairs, int* cnt, int* d_max,
+                      cudaStream_t st);
+// rows by decreasing hop count (stable): perm[place] = row, pinv[row] = place;
+// dim^2 comparisons
+void launch_hop_order(int dim, const int* cnt, int* perm, int* pinv, cudaStream_t st);
 void launch_hop_fill(int Ns, int n, int dim, int width, const int* words, const HopPair* d_pairs,
                      int npairs, int* src, double2* amp, cudaStream_t st);
 void launch_e1(int dim, const int* words, const E1Params& p, bool with_const, double2* e1,

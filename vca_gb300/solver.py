@@ -342,7 +342,8 @@ class VcaSolver:
         check(self.L.vca_gpu_set_chain_streams(int(n)))
 
     def set_hop_pairing(self, on: bool):
-        """Pair the chains' kernel's hop parities per quarter warp (default
+        """Pair the hop parities per quarter warp of up spaces of 128
+        configurations and more in the chains' kernel (default
         on; applies to the next set_hamiltonian)."""
         check(self.L.vca_gpu_set_hop_pairing(1 if on else 0))
 
