@@ -202,7 +202,8 @@ struct Ctx {
   double2* d_weights = nullptr;
   int* d_nexc = nullptr;
   bool poles_ready = false;
-  int ql_max_iter = 60;  // QL sweeps per eigenvalue before a chain is reported unconverged
+#define QL_MAX_ITER 60
+  int ql_max_iter = QL_MAX_ITER;  // QL sweeps per eigenvalue before a chain is reported unconverged
   bool omega_inverse_form = true;  // T=0 k-sum through G'^-1 + M at nodes with w <= 10
   ChainStore cstore{};
   int nelem = 0;
@@ -1768,8 +1769,8 @@ struct ChainSpec {
 // the same numbers.  (i,j) and (j,i) always share the chain of c_i + c_j; with a
 // real H also that of c_i + i c_j, since c_j + i c_i = i conj(c_i + i c_j) on
 // a real state (its re and im columns swap places, and every sum over the
-// pair is commutative).  Of 4L^2 - 2L channels 2L(L+1) chains (complex H:
-// L(3L+1)) are left to run.
+// pair is commutative).  Of 4L^2 - 2L channels 2L^2 chains (complex H:
+// L(3L-1)) are left to run.
 // Measured, whole solves: 4x3 cluster (one spin, 100 steps) 1541 -> 981 ms,
 // 3x3 161 -> 134 ms, BHZ (complex) 300 -> 281 ms.
 struct ChainKeys {
@@ -2553,20 +2554,46 @@ int omega_integral(double* out) {
 // vector vanished (n = 0; NaN in the reference, which the comparison skips)
 // add nothing.
 int chains_max_exc(double* out) {
-  RCHK(ensure_poles());
   const size_t nch = (size_t)g->nstore;
   double m = -DBL_MAX;
-  if (nch) {
+  std::vector<int> n(nch);
+  bool tops = nch && g->ql_max_iter == QL_MAX_ITER && chain_top_ok(g->cstore);
+  if (tops) {  // de = E_j - Ei is largest at the top of the chain's tridiagonal
+    Arena ar;
+    double *work, *d_top;
+    std::vector<double> top(nch), Ei(nch);
+    int rc = ar.alloc(&work, nch * 5 * (size_t)g->ld);
+    if (!rc) rc = ar.alloc(&d_top, nch);
+    if (!rc) launch_chain_top((int)nch, g->cstore, work, d_top, g->st);
+    cudaError_t e = cudaSuccess;
+    if (!rc) e = cudaMemcpyAsync(top.data(), d_top, sizeof(double) * nch, cudaMemcpyDeviceToHost, g->st);
+    if (!rc && e == cudaSuccess)
+      e = cudaMemcpyAsync(Ei.data(), g->cstore.Ei, sizeof(double) * nch, cudaMemcpyDeviceToHost, g->st);
+    if (!rc && e == cudaSuccess)
+      e = cudaMemcpyAsync(n.data(), g->cstore.n, sizeof(int) * nch, cudaMemcpyDeviceToHost, g->st);
+    if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(g->st);
+    ar.release();
+    if (rc) return rc;
+    CUCHK(e);
+    for (size_t ch = 0; ch < nch; ch++)
+      if (n[ch] > 0) {
+        tops = tops && std::isfinite(top[ch]);
+        m = std::max(m, top[ch] - Ei[ch]);
+      }
+    if (!tops) m = -DBL_MAX;
+  }
+  if (nch && !tops) {  // from the poles, whose QL reports what it cannot do
+    RCHK(ensure_poles());
     std::vector<double> p(nch * (size_t)g->ld);
-    std::vector<int> n(nch), sg(nch);
+    std::vector<int> sg(nch);
     CUCHK(cudaMemcpy(p.data(), g->d_poles, sizeof(double) * p.size(), cudaMemcpyDeviceToHost));
     CUCHK(cudaMemcpy(n.data(), g->d_nexc, sizeof(int) * nch, cudaMemcpyDeviceToHost));
     CUCHK(cudaMemcpy(sg.data(), g->cstore.isign, sizeof(int) * nch, cudaMemcpyDeviceToHost));
     for (size_t ch = 0; ch < nch; ch++)
       for (int j = 0; j < n[ch]; j++) m = std::max(m, sg[ch] * p[ch * g->ld + j]);  // poles = isign*de
-    for (const ChainRec& r : g->chains)
-      if (n[r.store] > 0 && n[r.store] < r.nlanc) m = std::max(m, -g->gs[r.state].e);
   }
+  for (const ChainRec& r : g->chains)
+    if (n[r.store] > 0 && n[r.store] < r.nlanc) m = std::max(m, -g->gs[r.state].e);
   *out = m;
   return VCA_OK;
 }

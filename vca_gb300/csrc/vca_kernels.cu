@@ -638,6 +638,39 @@ void launch_chain_poles(int nch, const ChainStore& cs, double* work, double* pol
   k_chain_poles<<<nblocks(nch, 32), 32, 0, st>>>(nch, cs, work, poles, weights, nexc, max_iter, fail);
 }
 
+// Largest eigenvalue of each chain's tridiagonal (the top of its poles), one
+// warp a chain: the lowest of -T (vca_tri.cuh; T and -T with the same
+// off-diagonal signs are similar).  work: 5*ld doubles per chain; ld <= TRI_MAX.
+// 3x3 cluster at finite T, 936 chains of 100 rows: 21.8 ms by the QL below,
+// which max_exc needs none of the rest of, -> 0.2 ms.  A chain with a value that
+// is not finite gives NaN.
+__global__ void __launch_bounds__(32) k_chain_top(ChainStore cs, double* work, double* top) {
+  __shared__ double a[TRI_MAX], b[TRI_MAX];
+  __shared__ float2 w[2 * TRI_MAX];
+  __shared__ double out[2];
+  const int ch = blockIdx.x, n = cs.n[ch];
+  bool finite = true;
+  for (int j = threadIdx.x; j < n; j += 32) {
+    a[j] = -cs.A[(int64_t)ch * cs.ld + j];
+    b[j] = j ? cs.B[(int64_t)ch * cs.ld + j] : 0.0;
+    finite = finite && isfinite(a[j]) && isfinite(b[j]);
+  }
+  if (!__all_sync(0xffffffffu, finite)) {
+    if (threadIdx.x == 0) top[ch] = nan("");
+    return;
+  }
+  __syncwarp();
+  if (n > 0) warp_tri_lowest(a, b, n, 0.0, 1.0, true, false, w, out, work + (int64_t)ch * 5 * cs.ld, out + 1);
+  __syncwarp();
+  if (threadIdx.x == 0) top[ch] = n > 0 ? -out[0] : 0.0;
+}
+bool chain_top_ok(const ChainStore& cs) { return cs.ld <= TRI_MAX; }
+void launch_chain_top(int nch, const ChainStore& cs, double* work, double* top, cudaStream_t st) {
+  if (nch <= 0) return;
+  COUNT_LAUNCH();
+  k_chain_top<<<nch, 32, 0, st>>>(cs, work, top);
+}
+
 // ---------------------------------------------------------------------------
 // Chain start vectors by gather: target row t, term (pos, coef): for c^dag
 // the target spin word must hold pos and the source is w - pos; for c it must

@@ -99,6 +99,10 @@ struct ChainStore {
 void launch_chain_store(int nch, const ChainMeta* meta, const double* A, const double* Bt, int ldab,
                         const double* norm2, const double2* wfac, const int* isign, double Ei, double boltz,
                         double zeta, const ChainStore& cs, int base, cudaStream_t st);
+// top[ch] = largest eigenvalue of the stored chain (0 when it is empty); work:
+// 5*ld doubles per chain
+bool chain_top_ok(const ChainStore& cs);
+void launch_chain_top(int nch, const ChainStore& cs, double* work, double* top, cudaStream_t st);
 // stored chains -> poles/weights (add_to_lanczos_gf_normal, VCA_GF_NORMAL.f90:970-1033);
 // work: 3*ld doubles per chain; *fail counts chains whose QL needed more
 // than max_iter sweeps for one eigenvalue
