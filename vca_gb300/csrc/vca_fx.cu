@@ -1968,9 +1968,24 @@ static void launch_hxv_fx_s_k(const SectorView& sv, const FxView& fv, int m, con
 // ---------------------------------------------------------------------------
 #define FXS_DW_ROWS 64
 #define FXS_DW_GRP 8
-template <int K>
-__global__ void __launch_bounds__(FX1_UP2_THREADS, 1) k_hxv_slab_up2(SectorView sv, FxView fv, int nslab,
-                                                                 const i64* __restrict__ X, i64* __restrict__ Y) {
+// (the alpha sums of the up part take a kilobyte of static shared memory)
+#define FXS_SMEM_UP2 (FX1_SMEM_MAX - 1024)
+#define FXS_DOT_ROWS (152 * 4)  // alpha partial rows of the slab-pair form
+// The down part runs first and writes its half; the up part adds it to its own
+// and, with x and the whole y at hand, forms the <X, Y> sums (apart): they go to
+// row blockIdx % FXS_DOT_ROWS of it (zeroed before) as 128-bit integers in two
+// words with the carry of the low one, exact in any order.  16 columns of the
+// 4x4 sector (9,8): 48.5 -> 46.0 ms; with the sums in the down part, which
+// has to read x for them, 51.5.
+__device__ __forceinline__ void fx_atomic_add128(i64* p, i128 v) {
+  const u64 lo = (u64)v;
+  const u64 old = atomicAdd((u64*)p, lo);
+  atomicAdd((u64*)p + 1, (u64)(v >> 64) + (old + lo < old ? 1ull : 0ull));
+}
+template <int K, bool APART>
+__global__ void __launch_bounds__(FX1_UP2_THREADS, 1) k_hxv_slab_up2(SectorView sv, FxView fv, int nslab, int m,
+                                                                 const i64* __restrict__ X, i64* __restrict__ Y,
+                                                                 i64* __restrict__ apart) {
   extern __shared__ __align__(16) unsigned char x1p_smem[];
   longlong2* xs = (longlong2*)x1p_smem;
   const int DU = sv.dimup, DD = sv.dimdw;
@@ -2001,11 +2016,13 @@ __global__ void __launch_bounds__(FX1_UP2_THREADS, 1) k_hxv_slab_up2(SectorView 
   const int nw = (DU + 31) >> 5;
   const i64 e1d = fv.dw_e1[idw];
   const unsigned wd = (unsigned)sv.dw_words[idw];
+  i128 ad0 = 0, ad1 = 0;
   for (int w = threadIdx.x >> 5; w < nw; w += FX1_UP2_THREADS / 32) {
     const int iup = w * 32 + lane;
     const bool row = iup < DU;
     const i64 eu = row ? fv.up_e1[iup] : 0;
     const unsigned wu = row ? (unsigned)sv.up_words[iup] : 0u;
+    const longlong2 yd = row ? __ldcg(Y2 + (int64_t)iup * 4) : make_longlong2(0ll, 0ll);  // the down half
     u64 A[K], B[K];
     up2_rounds<K>(fv, w, lane, DU, x1p_smem, A, B);
     if (!row) continue;
@@ -2015,8 +2032,37 @@ __global__ void __launch_bounds__(FX1_UP2_THREADS, 1) k_hxv_slab_up2(SectorView 
 #pragma unroll
     for (int k = 0; k < K; k++) p0 += (i128)fv.afx[k] * (i64)A[k], p1 += (i128)fv.afx[k] * (i64)B[k];
     const bool sh63 = fv.shift >= 1 && fv.shift <= 63;
-    __stcg(Y2 + (int64_t)iup * 4, make_longlong2((long long)rshift_round_u(p0, fv.shift, sh63),
-                                                 (long long)rshift_round_u(p1, fv.shift, sh63)));
+    const i64 ya = (i64)yd.x + rshift_round_u(p0, fv.shift, sh63), yb = (i64)yd.y + rshift_round_u(p1, fv.shift, sh63);
+    __stcg(Y2 + (int64_t)iup * 4, make_longlong2((long long)ya, (long long)yb));
+    if (APART) {
+      ad0 += (i128)xi.x * ya;
+      ad1 += (i128)xi.y * yb;
+    }
+  }
+  if (APART) {
+    __shared__ i128 red[FX1_UP2_THREADS / 32][2];
+    i128 adv[2] = {ad0, ad1};
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      u64 lo = (u64)adv[q];
+      i64 hi = (i64)(adv[q] >> 64);
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const u64 lo2 = __shfl_xor_sync(0xffffffffu, lo, off);
+        const i64 hi2 = __shfl_xor_sync(0xffffffffu, hi, off);
+        const u64 sl = lo + lo2;
+        hi = hi + hi2 + (sl < lo ? 1 : 0);
+        lo = sl;
+      }
+      if (lane == 0) red[threadIdx.x >> 5][q] = ((i128)hi << 64) | (i128)lo;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      i128 sum = 0;
+      for (int w = 0; w < FX1_UP2_THREADS / 32; w++) sum += red[w][threadIdx.x];
+      const int c = sl * FX_SLAB + 2 * pr + (int)threadIdx.x;
+      fx_atomic_add128(apart + 2 * ((int64_t)(rest % FXS_DOT_ROWS) * m + c), sum);
+    }
   }
 }
 
@@ -2040,7 +2086,6 @@ __global__ void __launch_bounds__(FXS_DW_ROWS * 4) k_hxv_slab_dw2(SectorView sv,
     if (idw >= DD) break;
     const int nd = sv.dw_cnt[idw], ndp = fv.dw_npos[idw];
     const int64_t own = (int64_t)idw * bstride;
-    const longlong2 y = __ldcg(Y2 + own);
     u64 A[K], B[K];
 #pragma unroll
     for (int k = 0; k < K; k++) A[k] = B[k] = 0;
@@ -2067,15 +2112,14 @@ __global__ void __launch_bounds__(FXS_DW_ROWS * 4) k_hxv_slab_dw2(SectorView sv,
 #pragma unroll
     for (int k = 0; k < K; k++) pa += (i128)fv.afx[k] * (i64)A[k], pb += (i128)fv.afx[k] * (i64)B[k];
     const bool sh63 = fv.shift >= 1 && fv.shift <= 63;
-    __stcg(Y2 + own, make_longlong2((long long)((i64)y.x + rshift_round_u(pa, fv.shift, sh63)),
-                                    (long long)((i64)y.y + rshift_round_u(pb, fv.shift, sh63))));
+    __stcg(Y2 + own, make_longlong2((long long)rshift_round_u(pa, fv.shift, sh63),
+                                    (long long)rshift_round_u(pb, fv.shift, sh63)));
   }
 }
 
-#define FXS_DOT_ROWS (152 * 4)  // alpha partial rows of the slab-pair form
 static bool hxv_fx_slab2_ok(const SectorView& sv, const FxView& fv, int m, bool warp_only) {
   return !warp_only && !fv.rows_permuted && fv.up_sched && fv.up_wround && fv.up_wgrp && fv.dw_npos &&
-         fx_pair_fits(sv.dimup) && m >= FX_SLAB && m % FX_SLAB == 0 &&
+         (size_t)(sv.dimup + FX1_ZERO_UNITS) * 16 <= FXS_SMEM_UP2 && m >= FX_SLAB && m % FX_SLAB == 0 &&
          (int64_t)sv.dimup * sv.dimdw >= FX1_MIN_DIM;
 }
 
@@ -2084,22 +2128,22 @@ static void launch_hxv_slab_k(const SectorView& sv, const FxView& fv, int m, con
                               cudaStream_t st) {
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_hxv_slab_up2<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, FX1_SMEM_MAX);
+    cudaFuncSetAttribute(k_hxv_slab_up2<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FXS_SMEM_UP2);
+    cudaFuncSetAttribute(k_hxv_slab_up2<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FXS_SMEM_UP2);
     attr = true;
   }
   const int nslab = m / FX_SLAB;
   const int DU = sv.dimup, DD = sv.dimdw;
   count_launch_external();
   count_launch_external();
-  k_hxv_slab_up2<K><<<DD * nslab * 4, FX1_UP2_THREADS, (size_t)(DU + FX1_ZERO_UNITS) * 16, st>>>(sv, fv, nslab, X, Y);
   const int nck = (DU + FXS_DW_ROWS - 1) / FXS_DW_ROWS, ngrp = (DD + FXS_DW_GRP - 1) / FXS_DW_GRP;
   k_hxv_slab_dw2<K><<<nck * nslab * ngrp, FXS_DW_ROWS * 4, 0, st>>>(sv, fv, nslab, X, Y);
+  const size_t shm = (size_t)(DU + FX1_ZERO_UNITS) * 16;
   if (apart) {  // exact int128 <X, Y> partials, FXS_DOT_ROWS rows of m
-    count_launch_external();
-    dim3 blk;
-    int ns;
-    slab_shape(m, blk, ns);
-    k_fx_dot<<<dim3(FXS_DOT_ROWS, ns, 1), blk, sizeof(i128) * 256, st>>>((int64_t)DU * DD, m, X, Y, apart);
+    cudaMemsetAsync(apart, 0, sizeof(i128) * FXS_DOT_ROWS * (size_t)m, st);
+    k_hxv_slab_up2<K, true><<<DD * nslab * 4, FX1_UP2_THREADS, shm, st>>>(sv, fv, nslab, m, X, Y, apart);
+  } else {
+    k_hxv_slab_up2<K, false><<<DD * nslab * 4, FX1_UP2_THREADS, shm, st>>>(sv, fv, nslab, m, X, Y, apart);
   }
 }
 
