@@ -10,7 +10,7 @@ from vca_gb300.solver import VcaSolver
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nup,ndw,m", [(8, 1, 16), (8, 2, 8), (5, 2, 24), (7, 3, 16)])
+@pytest.mark.parametrize("nup,ndw,m", [(8, 1, 16), (8, 2, 8), (5, 2, 24), (7, 3, 16), (8, 3, 8)])
 def test_alpha_is_the_exact_sum(nup, ndw, m):
     import torch
     pt = clusters.square(nx=4, ny=4, cdw=0.1, nspin=1, nkx=2, nky=2, ngfiter=4, omega_nodes=16)
