@@ -105,6 +105,24 @@ struct Arena {
   }
 };
 
+// Many tables in one allocation, each on a 256-byte boundary.
+struct TableAlloc {
+  std::vector<std::pair<char**, size_t>> want;  // where the pointer goes, its offset
+  size_t bytes = 0;
+  template <typename T>
+  void add(T** p, size_t n) {
+    want.push_back({(char**)p, bytes});
+    bytes += (n * sizeof(T) + 255) / 256 * 256;
+  }
+  int alloc(Arena& ar) {
+    char* base;
+    const int rc = ar.alloc(&base, bytes);
+    if (rc) return rc;
+    for (auto& w : want) *w.first = base + w.second;
+    return VCA_OK;
+  }
+};
+
 struct GState {
   int sector;
   double e;
@@ -414,6 +432,7 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
   g->real_model = real;
   g->rs_split = 1;
   g->rs_diag_im = 0;
+  TabSet tabs[2] = {};
   const int LC = c.Nlat * c.Norb;
   for (int set = 0; set < nsets; set++) {
     const int sidx = (set == 0) ? 0 : c.Nspin - 1;
@@ -489,28 +508,42 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
     }
     g->sp[set].assign(g->Ns + 1, SpinSpace());
     // every filling's counts, then their widths in one read
+    TabSet& ts = tabs[set];
+    ts.n = g->Ns + 1;
     int widths[VCA_MAX_NS + 1];
     CUCHK(cudaMemsetAsync(g->d_iscratch, 0, sizeof(int) * (g->Ns + 1), g->st));
+    TableAlloc counts, rest;
     for (int n = 0; n <= g->Ns; n++) {
-      SpinSpace& S = g->sp[set][n];
-      S.n = n;
-      S.dim = g->dimn[n];
-      S.words = g->words[n];
-      RCHK(g->ham.alloc(&S.cnt, S.dim));
-      launch_hop_count(S.dim, S.words, g->d_pairs[set], (int)pairs.size(), S.cnt, g->d_iscratch + n, g->st);
+      TabSpace& T = ts.s[n];
+      T.dim = g->dimn[n];
+      T.words = g->words[n];
+      counts.add(&T.cnt, T.dim);
     }
+    RCHK(counts.alloc(g->ham));
+    launch_tab_count(ts, g->d_pairs[set], (int)pairs.size(), g->d_iscratch, g->st);
     CUCHK(cudaMemcpyAsync(widths, g->d_iscratch, sizeof(int) * (g->Ns + 1), cudaMemcpyDeviceToHost, g->st));
     CUCHK(cudaStreamSynchronize(g->st));
     for (int n = 0; n <= g->Ns; n++) {
+      TabSpace& T = ts.s[n];
+      T.width = widths[n];
+      rest.add(&T.src, (size_t)T.width * T.dim);
+      rest.add(&T.amp, (size_t)T.width * T.dim);
+      rest.add(&T.e1, T.dim);
+    }
+    RCHK(rest.alloc(g->ham));
+    launch_tab_fill(ts, g->d_pairs[set], (int)pairs.size(), ep, g->st);
+    CUCHK(cudaGetLastError());
+    for (int n = 0; n <= g->Ns; n++) {
+      const TabSpace& T = ts.s[n];
       SpinSpace& S = g->sp[set][n];
-      S.width = widths[n];
-      RCHK(g->ham.alloc(&S.src, (size_t)S.width * S.dim));
-      RCHK(g->ham.alloc(&S.amp, (size_t)S.width * S.dim));
-      RCHK(g->ham.alloc(&S.e1, S.dim));
-      launch_hop_fill(g->Ns, n, S.dim, S.width, S.words, g->d_pairs[set], (int)pairs.size(), S.src, S.amp,
-                      g->st);
-      launch_e1(S.dim, S.words, ep, false, S.e1, g->st);
-      CUCHK(cudaGetLastError());
+      S.n = n;
+      S.dim = T.dim;
+      S.width = T.width;
+      S.words = g->words[n];
+      S.cnt = T.cnt;
+      S.src = T.src;
+      S.amp = T.amp;
+      S.e1 = T.e1;
     }
   }
   if (nsets == 1) g->sp[1] = g->sp[0];
@@ -583,47 +616,63 @@ int set_hamiltonian(const double* Hloc, const double* bath_h, const double* bath
         g->fx_sched[set].assign(g->Ns + 1, nullptr);
         g->fx_wround[set].assign(g->Ns + 1, nullptr);
         g->fx_wgrp[set].assign(g->Ns + 1, nullptr);
+        TabSet& ts = tabs[set];
+        TableAlloc ta;
+        for (int n = 0; n <= g->Ns; n++) {
+          TabSpace& T = ts.s[n];
+          const size_t hops = (size_t)T.width * T.dim;
+          ta.add(&T.hop, hops);
+          ta.add(&T.code, hops);
+          ta.add(&T.npos, T.dim);
+          ta.add(&T.e1fx, T.dim);
+          ta.add(&T.perm, T.dim);
+          ta.add(&T.pinv, T.dim);
+          ta.add(&T.phop, hops);
+          ta.add(&T.rhop, hops);
+          ta.add(&T.pcnt, T.dim);
+          ta.add(&T.pnpos, T.dim);
+          ta.add(&T.pword, T.dim);
+          ta.add(&T.pe1, T.dim);
+        }
+        RCHK(ta.alloc(g->ham));
+        launch_tab_fx(ts, d_cls, fb.K, fs.A, g->st);
+        // rows by decreasing hop count (stable), for warps of equal loop length; the
+        // device's dim^2 comparisons against a sort on the host and its copies
+        // (100 us a space): 40 us at the 12,870 rows of the 4x4 cluster
+        launch_tab_order(ts, g->st);
+        for (int n = 0; n <= g->Ns; n++) {
+          const TabSpace& T = ts.s[n];
+          if (T.dim <= TAB_ORDER_MAX) continue;
+          std::vector<int> cnt(T.dim), perm(T.dim), pinv(T.dim);
+          CUCHK(cudaMemcpyAsync(cnt.data(), T.cnt, sizeof(int) * T.dim, cudaMemcpyDeviceToHost, g->st));
+          CUCHK(cudaStreamSynchronize(g->st));
+          for (int r = 0; r < T.dim; r++) perm[r] = r;
+          std::stable_sort(perm.begin(), perm.end(), [&](int x, int y) { return cnt[x] > cnt[y]; });
+          for (int r = 0; r < T.dim; r++) pinv[perm[r]] = r;
+          CUCHK(cudaMemcpyAsync(T.perm, perm.data(), sizeof(int) * T.dim, cudaMemcpyHostToDevice, g->st));
+          CUCHK(cudaMemcpyAsync(T.pinv, pinv.data(), sizeof(int) * T.dim, cudaMemcpyHostToDevice, g->st));
+          CUCHK(cudaStreamSynchronize(g->st));  // host vectors go out of scope
+        }
+        launch_tab_perm(ts, g->st);
+        CUCHK(cudaGetLastError());
         int64_t partner = 0;  // largest spin space the other role can take
         for (int n = 0; n <= g->Ns; n++) partner = std::max<int64_t>(partner, g->sp[nsets - 1 - set][n].dim);
         for (int n = 0; n <= g->Ns; n++) {
           SpinSpace& S = g->sp[set][n];
-          RCHK(g->ham.alloc(&g->fx_hop[set][n], (size_t)S.width * S.dim));
-          launch_fx_pack(S.dim, S.width, S.src, S.amp, d_cls, fb.K, g->fx_hop[set][n], g->st);
-          RCHK(g->ham.alloc(&g->fx_npos[set][n], S.dim));
-          launch_fx_sign_sort(S.dim, S.width, S.cnt, g->fx_hop[set][n], g->fx_npos[set][n], g->st);
-          RCHK(g->ham.alloc(&g->fx_perm[set][n], S.dim));
-          RCHK(g->ham.alloc(&g->fx_ptab[set][n].pinv, S.dim));
-          // rows by decreasing hop count (stable), for warps of equal loop length; the
-          // device's dim^2 comparisons against a sort on the host and its copies
-          // (100 us a space): 40 us at the 12,870 rows of the 4x4 cluster
-          if (S.dim <= 1 << 14) {
-            launch_hop_order(S.dim, S.cnt, g->fx_perm[set][n], g->fx_ptab[set][n].pinv, g->st);
-          } else {
-            std::vector<int> cnt(S.dim), perm(S.dim);
-            if (S.dim) CUCHK(cudaMemcpy(cnt.data(), S.cnt, sizeof(int) * S.dim, cudaMemcpyDeviceToHost));
-            for (int r = 0; r < S.dim; r++) perm[r] = r;
-            std::stable_sort(perm.begin(), perm.end(), [&](int x, int y) { return cnt[x] > cnt[y]; });
-            std::vector<int> pinv(S.dim);
-            for (int r = 0; r < S.dim; r++) pinv[perm[r]] = r;
-            if (S.dim) {
-              CUCHK(cudaMemcpy(g->fx_perm[set][n], perm.data(), sizeof(int) * S.dim, cudaMemcpyHostToDevice));
-              CUCHK(cudaMemcpy(g->fx_ptab[set][n].pinv, pinv.data(), sizeof(int) * S.dim, cudaMemcpyHostToDevice));
-            }
-          }
-          RCHK(g->ham.alloc(&g->fx_code[set][n], (size_t)S.width * S.dim));
-          RCHK(g->ham.alloc(&g->fx_e1[set][n], S.dim));
-          launch_fx_codes(S.dim, S.width, S.amp, d_cls, fb.K, g->fx_code[set][n], g->st);
-          launch_fx_e1(S.dim, S.e1, fs.A, g->fx_e1[set][n], g->st);
+          const TabSpace& T = ts.s[n];
+          g->fx_hop[set][n] = T.hop;
+          g->fx_npos[set][n] = T.npos;
+          g->fx_perm[set][n] = T.perm;
+          g->fx_code[set][n] = T.code;
+          g->fx_e1[set][n] = T.e1fx;
           Ctx::PermTabs& pt = g->fx_ptab[set][n];
-          RCHK(g->ham.alloc(&pt.hop, (size_t)S.width * S.dim));
-          RCHK(g->ham.alloc(&pt.rhop, (size_t)S.width * S.dim));
-          RCHK(g->ham.alloc(&pt.cnt, S.dim));
-          RCHK(g->ham.alloc(&pt.npos, S.dim));
-          RCHK(g->ham.alloc(&pt.word, S.dim));
-          RCHK(g->ham.alloc(&pt.e1, S.dim));
-          launch_fx_perm_tables(S.dim, S.width, g->fx_perm[set][n], pt.pinv, g->fx_hop[set][n], S.cnt,
-                                g->fx_npos[set][n], S.words, g->fx_e1[set][n], pt.hop, pt.rhop, pt.cnt, pt.npos,
-                                pt.word, pt.e1, g->st);
+          pt.pinv = T.pinv;
+          pt.hop = T.phop;
+          pt.rhop = T.rhop;
+          pt.cnt = T.pcnt;
+          pt.npos = T.pnpos;
+          pt.word = T.pword;
+          pt.e1 = T.pe1;
           if (S.dim >= 128 && (size_t)S.dim * FX_SLAB * sizeof(i64) <= 200 * 1024 && g->rhop_order) {
             // the position-ordered kernel's up block fits: pair its rows' hop parities
             // (smaller spaces' chains run resident, vca_resident.cuh)

@@ -64,37 +64,6 @@ __device__ __forceinline__ double i128_to_double(i128 v, int scale_exp) {
 }
 
 // ---------------------------------------------------------------------------
-// tables
-// ---------------------------------------------------------------------------
-__global__ void k_fx_codes(int64_t n, const double2* amp, const double* classes, int K, signed char* code) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const double a = amp[t].x;
-    const double mag = fabs(a);
-    int cls = 0;
-    for (int k = 0; k < K; k++)
-      if (classes[k] == mag) cls = k;
-    code[t] = (signed char)(cls | (a < 0.0 ? 0x80 : 0));
-  }
-}
-void launch_fx_codes(int dim, int width, const double2* amp, const double* classes, int K,
-                     signed char* code, cudaStream_t st) {
-  count_launch_external();
-  int64_t n = (int64_t)dim * width;
-  if (n == 0) return;
-  k_fx_codes<<<nblk_fx(n, 256), 256, 0, st>>>(n, amp, classes, K, code);
-}
-
-__global__ void k_fx_e1(int dim, const double2* e1, int A, i64* e1fx) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < dim; r += gridDim.x * blockDim.x)
-    e1fx[r] = __double2ll_rn(ldexp(e1[r].x, A));
-}
-void launch_fx_e1(int dim, const double2* e1, int A, i64* e1fx, cudaStream_t st) {
-  count_launch_external();
-  k_fx_e1<<<nblk_fx(dim, 256), 256, 0, st>>>(dim, e1, A, e1fx);
-}
-
-// ---------------------------------------------------------------------------
 // H x v in fixed point.  Same row/column mapping as the FP64 kernel; every hop
 // is an exact int64 add into the accumulator of its amplitude class.
 // ---------------------------------------------------------------------------
@@ -1073,75 +1042,6 @@ void launch_fx_start_raw(int64_t n, uint64_t seed, int isector, i64* R, cudaStre
 // ---------------------------------------------------------------------------
 // Packed hop words and the warp-per-row H x v for column batches.
 // ---------------------------------------------------------------------------
-__global__ void k_fx_pack(int64_t n, const int* src, const double2* amp, const double* classes, int K,
-                          unsigned* hop) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const double a = amp[t].x;
-    const double mag = fabs(a);
-    unsigned cls = 0;
-    for (int k = 0; k < K; k++)
-      if (classes[k] == mag) cls = (unsigned)k;
-    hop[t] = ((unsigned)src[t] & 0xFFFFFFu) | (cls << 24) | (a < 0.0 ? 0x80000000u : 0u);
-  }
-}
-void launch_fx_pack(int dim, int width, const int* src, const double2* amp, const double* classes, int K,
-                    unsigned* hop, cudaStream_t st) {
-  count_launch_external();
-  const int64_t n = (int64_t)dim * width;
-  if (n == 0) return;
-  k_fx_pack<<<nblk_fx(n, 256), 256, 0, st>>>(n, src, amp, classes, K, hop);
-}
-
-// In-place partition of each row's hop words, positive amplitudes first;
-// npos[row] = their count.  The fixed-point sums are exact, so the order of
-// a row's hops does not change any result.
-__global__ void k_fx_sign_sort(int dim, int width, const int* cnt, unsigned* hop, int* npos) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= dim) return;
-  int i = 0, j = cnt[r] - 1;
-  while (i <= j) {
-    const unsigned a = hop[r + (int64_t)i * dim];
-    if (!(a >> 31)) { i++; continue; }
-    const unsigned b = hop[r + (int64_t)j * dim];
-    hop[r + (int64_t)i * dim] = b;
-    hop[r + (int64_t)j * dim] = a;
-    j--;
-  }
-  npos[r] = i;
-}
-void launch_fx_sign_sort(int dim, int width, const int* cnt, unsigned* hop, int* npos, cudaStream_t st) {
-  if (dim == 0) return;
-  count_launch_external();
-  k_fx_sign_sort<<<(dim + 127) / 128, 128, 0, st>>>(dim, width, cnt, hop, npos);
-}
-
-__global__ void k_fx_perm_tables(int dim, int width, const int* perm, const int* pinv, const unsigned* hop,
-                                 const int* cnt, const int* npos, const int* words, const i64* e1, unsigned* phop,
-                                 unsigned* rhop, int* pcnt, int* pnpos, int* pword, i64* pe1) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= dim) return;
-  const int r = perm[i];
-  pcnt[i] = cnt[r];
-  pnpos[i] = npos[r];
-  pword[i] = words[r];
-  pe1[i] = e1[r];
-  for (int h = 0; h < width; h++) {  // source as its first swizzled 16-byte unit (see fxs_unit)
-    const unsigned hw = hop[(int64_t)h * dim + r];
-    const unsigned src = hw & 0xFFFFFFu;
-    phop[(int64_t)h * dim + i] = (src * 4u + ((src >> 1) & 3u)) | (hw & 0xFF000000u);
-    rhop[(int64_t)h * dim + i] = (h < cnt[r] ? (unsigned)pinv[src] : 0u) | (hw & 0xFF000000u);
-  }
-}
-void launch_fx_perm_tables(int dim, int width, const int* perm, const int* pinv, const unsigned* hop,
-                           const int* cnt, const int* npos, const int* words, const i64* e1, unsigned* phop,
-                           unsigned* rhop, int* pcnt, int* pnpos, int* pword, i64* pe1, cudaStream_t st) {
-  if (dim == 0) return;
-  count_launch_external();
-  k_fx_perm_tables<<<(dim + 127) / 128, 128, 0, st>>>(dim, width, perm, pinv, hop, cnt, npos, words, e1, phop,
-                                                      rhop, pcnt, pnpos, pword, pe1);
-}
-
 __global__ void k_fx_pack16(int dim, int width, const int* cnt, const int* npos, const unsigned* rhop, unsigned* p16,
                             unsigned short* n16) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

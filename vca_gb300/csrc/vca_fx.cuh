@@ -102,15 +102,6 @@ __host__ __device__ __forceinline__ int64_t fx_off(int64_t D, int W, int64_t i, 
 __host__ __device__ inline int fx_p16_width(int width) { return (width + 1) / 2; }
 void launch_fx_pack16(int dim, int width, const int* cnt, const int* npos, const unsigned* rhop, unsigned* p16,
                       unsigned short* n16, cudaStream_t st);
-// up-spin tables in the order of perm (see FxView::up_phop)
-void launch_fx_perm_tables(int dim, int width, const int* perm, const int* pinv, const unsigned* hop,
-                           const int* cnt, const int* npos, const int* words, const i64* e1, unsigned* phop,
-                           unsigned* rhop, int* pcnt, int* pnpos, int* pword, i64* pe1, cudaStream_t st);
-// partition each row's hop words positive-first in place; npos[row] counts them
-void launch_fx_sign_sort(int dim, int width, const int* cnt, unsigned* hop, int* npos, cudaStream_t st);
-// packed hop words src | class<<24 | sign<<31 from the FP64 tables
-void launch_fx_pack(int dim, int width, const int* src, const double2* amp, const double* classes, int K,
-                    unsigned* hop, cudaStream_t st);
 // Y = H X on a slab-major column batch (m >= 16), one warp per row and
 // 128-column slice; with apart != nullptr also the exact alpha partials
 // <X,Y> per (row block, column), hxv_fx_w_rowblocks(D) rows of m int128
@@ -128,11 +119,6 @@ int hxv_fx_cols_rows(const SectorView& sv, const FxView& fv, int m, bool warp_on
 bool hxv_fx_r_ok(const SectorView& sv, const FxView& fv, int m);
 void launch_hxv_fx_cols(const SectorView& sv, const FxView& fv, int m, const i64* X, i64* Y, i64* apart,
                         bool warp_only, cudaStream_t st);
-// per-hop class/sign codes from the FP64 amplitude tables
-void launch_fx_codes(int dim, int width, const double2* amp, const double* classes, int K,
-                     signed char* code, cudaStream_t st);
-// FP64 one-body table -> fixed point
-void launch_fx_e1(int dim, const double2* e1, int A, i64* e1fx, cudaStream_t st);
 // Bank schedule of the paired-column staged up kernel.  Rows are taken in
 // warps of 32, and a warp's hops in groups g = 2*class + (amplitude < 0);
 // group g of warp w gets wgrp[w*2K + g] rounds (the most hops of that group

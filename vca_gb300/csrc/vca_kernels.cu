@@ -85,108 +85,155 @@ void launch_build_words(int Ns, int n, int dim, int* words, cudaStream_t st) {
 // spH0ups/spH0dws of VCA_HAMILTONIAN/stored/H_cluster_up.f90 (cluster :1-28,
 // bath :30-55, hybridisation :57-86) enumerated by target instead of source.
 // ---------------------------------------------------------------------------
-__global__ void k_hop_count(int dim, const int* words, const HopPair* pairs, int npairs, int* cnt,
-                            int* gmax) {
-  int local_max = 0;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < dim; r += gridDim.x * blockDim.x) {
-    unsigned w = (unsigned)words[r];
-    int c = 0;
-    for (int q = 0; q < npairs; q++) {
-      HopPair p = pairs[q];
-      if (((w >> p.i) & 1u) && !((w >> p.j) & 1u)) c++;
-    }
-    cnt[r] = c;
-    local_max = max(local_max, c);
-  }
-  atomicMax(gmax, local_max);
-}
-void launch_hop_count(int dim, const int* words, const HopPair* d_pairs, int npairs, int* cnt, int* d_max,
-                      cudaStream_t st) {
-  COUNT_LAUNCH();
-  k_hop_count<<<nblocks(dim, 256), 256, 0, st>>>(dim, words, d_pairs, npairs, cnt, d_max);
+static dim3 tab_grid(const TabSet& t, int threads, int most) {
+  int dmax = 1;
+  for (int i = 0; i < t.n; i++) dmax = std::max(dmax, std::min(t.s[i].dim, most));
+  return dim3((dmax + threads - 1) / threads, t.n, 1);
 }
 
-// Rows by decreasing hop count, stable: each row's place is the number of
-// rows before it, counted in chunks of rows staged in shared memory.
-__global__ void k_hop_order(int dim, const int* cnt, int* perm, int* pinv) {
+__global__ void __launch_bounds__(256) k_tab_count(const __grid_constant__ TabSet t, const HopPair* pairs, int npairs,
+                                                   int* gmax) {
+  const TabSpace& s = t.s[blockIdx.y];
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  int c = 0;
+  if (r < s.dim) {
+    const unsigned w = (unsigned)s.words[r];
+    for (int q = 0; q < npairs; q++) {
+      const HopPair p = pairs[q];
+      if (((w >> p.i) & 1u) && !((w >> p.j) & 1u)) c++;
+    }
+    s.cnt[r] = c;
+  }
+  const int most = __reduce_max_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(gmax + blockIdx.y, most);
+}
+void launch_tab_count(const TabSet& t, const HopPair* d_pairs, int npairs, int* d_max, cudaStream_t st) {
+  COUNT_LAUNCH();
+  k_tab_count<<<tab_grid(t, 256, 1 << 30), 256, 0, st>>>(t, d_pairs, npairs, d_max);
+}
+
+// Each row's place is the number of rows before it, counted in chunks of rows
+// staged in shared memory.
+__global__ void __launch_bounds__(128) k_tab_order(const __grid_constant__ TabSet t) {
+  const TabSpace& s = t.s[blockIdx.y];
+  const int dim = s.dim;
+  if (dim > TAB_ORDER_MAX || (int)(blockIdx.x * blockDim.x) >= dim) return;  // the whole block
   __shared__ int c[1024];
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  const int mine = r < dim ? cnt[r] : 0;
+  const int mine = r < dim ? s.cnt[r] : 0;
   int q = 0;
   for (int i0 = 0; i0 < dim; i0 += 1024) {
     const int n = min(1024, dim - i0);
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) c[i] = cnt[i0 + i];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) c[i] = s.cnt[i0 + i];
     __syncthreads();
     for (int i = 0; i < n; i++) q += c[i] > mine || (c[i] == mine && i0 + i < r);
   }
   if (r < dim) {
-    perm[q] = r;
-    pinv[r] = q;
+    s.perm[q] = r;
+    s.pinv[r] = q;
   }
 }
-void launch_hop_order(int dim, const int* cnt, int* perm, int* pinv, cudaStream_t st) {
-  if (dim <= 0) return;
+void launch_tab_order(const TabSet& t, cudaStream_t st) {
   COUNT_LAUNCH();
-  k_hop_order<<<(dim + 127) / 128, 128, 0, st>>>(dim, cnt, perm, pinv);
+  k_tab_order<<<tab_grid(t, 128, TAB_ORDER_MAX), 128, 0, st>>>(t);
 }
 
-__global__ void k_hop_fill(int dim, int width, const int* words, const HopPair* pairs, int npairs,
-                           int* src, double2* amp) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < dim; r += gridDim.x * blockDim.x) {
-    unsigned w = (unsigned)words[r];
-    int c = 0;
-    for (int q = 0; q < npairs && c < width; q++) {
-      HopPair p = pairs[q];
-      if (!(((w >> p.i) & 1u) && !((w >> p.j) & 1u))) continue;
-      unsigned ws = (w ^ (1u << p.i)) | (1u << p.j);
-      double sg1 = parity(ws & ((1u << p.j) - 1u));
-      unsigned k1 = ws & ~(1u << p.j);
-      double sg2 = parity(k1 & ((1u << p.i) - 1u));
-      double sg = sg1 * sg2;
-      src[(int64_t)c * dim + r] = rank_word(ws);
-      amp[(int64_t)c * dim + r] = make_double2(p.re * sg, p.im * sg);
-      c++;
-    }
-    for (; c < width; c++) {  // padding never read (cnt[r] bounds the loop)
-      src[(int64_t)c * dim + r] = 0;
-      amp[(int64_t)c * dim + r] = make_double2(0.0, 0.0);
-    }
+// hops, and the one-body + same-spin energy of a word (H_cluster_local.f90:19-25,
+// 46-55,59-76,84-92)
+__global__ void __launch_bounds__(256) k_tab_fill(const __grid_constant__ TabSet t, const HopPair* pairs, int npairs,
+                                                  const __grid_constant__ E1Params p) {
+  const TabSpace& s = t.s[blockIdx.y];
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= s.dim) return;
+  const unsigned w = (unsigned)s.words[r];
+  int c = 0;
+  for (int q = 0; q < npairs && c < s.width; q++) {
+    const HopPair h = pairs[q];
+    if (!(((w >> h.i) & 1u) && !((w >> h.j) & 1u))) continue;
+    const unsigned ws = (w ^ (1u << h.i)) | (1u << h.j);
+    const double sg1 = parity(ws & ((1u << h.j) - 1u));
+    const unsigned k1 = ws & ~(1u << h.j);
+    const double sg2 = parity(k1 & ((1u << h.i) - 1u));
+    const double sg = sg1 * sg2;
+    s.src[(int64_t)c * s.dim + r] = rank_word(ws);
+    s.amp[(int64_t)c * s.dim + r] = make_double2(h.re * sg, h.im * sg);
+    c++;
   }
+  for (; c < s.width; c++) {  // padding never read (cnt[r] bounds the loop)
+    s.src[(int64_t)c * s.dim + r] = 0;
+    s.amp[(int64_t)c * s.dim + r] = make_double2(0.0, 0.0);
+  }
+  double er = 0.0, ei = 0.0;
+  for (unsigned x = w; x; x &= x - 1) {
+    const int b = __ffs(x) - 1;
+    er += p.eps[b].x;
+    ei += p.eps[b].y;
+  }
+  int same = 0;
+  for (int o = 0; o < p.norb; o++)
+    for (int q = o + 1; q < p.norb; q++) same += __popc(w & p.omask[o] & (w >> (q - o)));
+  er += p.upar * same;
+  s.e1[r] = make_double2(er, ei);
 }
-void launch_hop_fill(int Ns, int n, int dim, int width, const int* words, const HopPair* d_pairs,
-                     int npairs, int* src, double2* amp, cudaStream_t st) {
+void launch_tab_fill(const TabSet& t, const HopPair* d_pairs, int npairs, const E1Params& p, cudaStream_t st) {
   COUNT_LAUNCH();
-  (void)Ns;
-  (void)n;
-  if (width == 0) return;
-  k_hop_fill<<<nblocks(dim, 256), 256, 0, st>>>(dim, width, words, d_pairs, npairs, src, amp);
+  k_tab_fill<<<tab_grid(t, 256, 1 << 30), 256, 0, st>>>(t, d_pairs, npairs, p);
 }
 
-// one-body + same-spin energy of a word (H_cluster_local.f90:19-25,46-55,59-76,84-92)
-__global__ void k_e1(int dim, const int* words, E1Params p, int with_const, double2* e1) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < dim; r += gridDim.x * blockDim.x) {
-    unsigned w = (unsigned)words[r];
-    double er = 0.0, ei = 0.0;
-    unsigned x = w;
-    while (x) {
-      int b = __ffs(x) - 1;
-      er += p.eps[b].x;
-      ei += p.eps[b].y;
-      x &= x - 1;
-    }
-    int same = 0;
-    for (int o = 0; o < p.norb; o++)
-      for (int q = o + 1; q < p.norb; q++) same += __popc(w & p.omask[o] & (w >> (q - o)));
-    er += p.upar * same;
-    if (with_const) { er += p.cst.x; ei += p.cst.y; }
-    e1[r] = make_double2(er, ei);
+// A row's hops to packed words and codes, then its words parted in place,
+// positive amplitudes first (the fixed-point sums are exact, so the order of a
+// row's hops changes no result).
+__global__ void __launch_bounds__(128) k_tab_fx(const __grid_constant__ TabSet t, const double* classes, int K, int A) {
+  const TabSpace& s = t.s[blockIdx.y];
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= s.dim) return;
+  for (int h = 0; h < s.width; h++) {
+    const int64_t q = (int64_t)h * s.dim + r;
+    const double a = s.amp[q].x;
+    const double mag = fabs(a);
+    unsigned cls = 0;
+    for (int k = 0; k < K; k++)
+      if (classes[k] == mag) cls = (unsigned)k;
+    s.code[q] = (signed char)((int)cls | (a < 0.0 ? 0x80 : 0));
+    s.hop[q] = ((unsigned)s.src[q] & 0xFFFFFFu) | (cls << 24) | (a < 0.0 ? 0x80000000u : 0u);
+  }
+  int i = 0, j = s.cnt[r] - 1;
+  while (i <= j) {
+    const unsigned a = s.hop[r + (int64_t)i * s.dim];
+    if (!(a >> 31)) { i++; continue; }
+    const unsigned b = s.hop[r + (int64_t)j * s.dim];
+    s.hop[r + (int64_t)i * s.dim] = b;
+    s.hop[r + (int64_t)j * s.dim] = a;
+    j--;
+  }
+  s.npos[r] = i;
+  s.e1fx[r] = __double2ll_rn(ldexp(s.e1[r].x, A));
+}
+void launch_tab_fx(const TabSet& t, const double* classes, int K, int A, cudaStream_t st) {
+  COUNT_LAUNCH();
+  k_tab_fx<<<tab_grid(t, 128, 1 << 30), 128, 0, st>>>(t, classes, K, A);
+}
+
+__global__ void __launch_bounds__(128) k_tab_perm(const __grid_constant__ TabSet t) {
+  const TabSpace& s = t.s[blockIdx.y];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= s.dim) return;
+  const int r = s.perm[i], n = s.cnt[r];
+  s.pcnt[i] = n;
+  s.pnpos[i] = s.npos[r];
+  s.pword[i] = s.words[r];
+  s.pe1[i] = s.e1fx[r];
+  for (int h = 0; h < s.width; h++) {  // source as its first swizzled 16-byte unit (see fxs_unit)
+    const unsigned hw = s.hop[(int64_t)h * s.dim + r];
+    const unsigned src = hw & 0xFFFFFFu;
+    s.phop[(int64_t)h * s.dim + i] = (src * 4u + ((src >> 1) & 3u)) | (hw & 0xFF000000u);
+    s.rhop[(int64_t)h * s.dim + i] = (h < n ? (unsigned)s.pinv[src] : 0u) | (hw & 0xFF000000u);
   }
 }
-void launch_e1(int dim, const int* words, const E1Params& p, bool with_const, double2* e1,
-               cudaStream_t st) {
+void launch_tab_perm(const TabSet& t, cudaStream_t st) {
   COUNT_LAUNCH();
-  k_e1<<<nblocks(dim, 256), 256, 0, st>>>(dim, words, p, with_const ? 1 : 0, e1);
+  k_tab_perm<<<tab_grid(t, 128, 1 << 30), 128, 0, st>>>(t);
 }
 
 // ---------------------------------------------------------------------------

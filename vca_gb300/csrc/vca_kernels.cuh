@@ -18,21 +18,47 @@ struct HopPair {     // amplitude of c^dag_i c_j for one spin (i != j), 0-based 
 };
 struct E1Params {    // one-body + same-spin diagonal energy of a spin word
   double2 eps[VCA_MAX_NS];   // per-level energy (incl. -xmu and Hartree shifts)
-  double2 cst;               // constant added once (carried by the up word)
   double upar;               // (Ust - Jh), same site, parallel spins
   int norb;
   unsigned int omask[VCA_MAX_NORB];
 };
-// hops per target word; *d_max gains the ELL width (most hops of a word)
-void launch_hop_count(int dim, const int* words, const HopPair* d_pairs, int npairs, int* cnt, int* d_max,
-                      cudaStream_t st);
-// rows by decreasing hop count (stable): perm[place] = row, pinv[row] = place;
-// dim^2 comparisons
-void launch_hop_order(int dim, const int* cnt, int* perm, int* pinv, cudaStream_t st);
-void launch_hop_fill(int Ns, int n, int dim, int width, const int* words, const HopPair* d_pairs,
-                     int npairs, int* src, double2* amp, cudaStream_t st);
-void launch_e1(int dim, const int* words, const E1Params& p, bool with_const, double2* e1,
-               cudaStream_t st);
+// The tables of one spin set's fillings, and the kernels that fill them, each one
+// launch over all fillings (blockIdx.y).  Small clusters are bound by launches: with
+// one per filling and table, and a table an allocation, the 2x2 cluster's two sets
+// took 90 launches and 160 allocations; now 10 and 6, whole solve 1.64 -> 1.29 ms
+// (4-site chain 1.63 -> 1.44 ms).
+struct TabSpace {
+  int dim, width;
+  const int* words;
+  int *cnt, *src;       // hops per target word; [width*dim], k-major
+  double2 *amp, *e1;
+  // fixed point: packed hop words src | class<<24 | sign<<31, each row's positive
+  // ones first (npos of them); class/sign codes in amp's order; one-body energies
+  unsigned* hop;
+  signed char* code;
+  int* npos;
+  long long* e1fx;
+  int *perm, *pinv;     // rows by decreasing hop count (stable): place -> row, row -> place
+  // the tables in perm's order (see FxView::up_phop)
+  unsigned *phop, *rhop;
+  int *pcnt, *pnpos, *pword;
+  long long* pe1;
+};
+struct TabSet {
+  int n;                // fillings
+  TabSpace s[VCA_MAX_NS + 1];
+};
+#define TAB_ORDER_MAX (1 << 14)  // rows whose order the device finds (dim^2 comparisons)
+// cnt, and d_max[filling] gains the most hops of a word (the ELL width)
+void launch_tab_count(const TabSet& t, const HopPair* d_pairs, int npairs, int* d_max, cudaStream_t st);
+// src, amp, e1
+void launch_tab_fill(const TabSet& t, const HopPair* d_pairs, int npairs, const E1Params& p, cudaStream_t st);
+// hop, code, npos, e1fx from the FP64 tables (A: scale of e1fx)
+void launch_tab_fx(const TabSet& t, const double* classes, int K, int A, cudaStream_t st);
+// perm, pinv of the fillings of at most TAB_ORDER_MAX rows
+void launch_tab_order(const TabSet& t, cudaStream_t st);
+// phop, rhop, pcnt, pnpos, pword, pe1
+void launch_tab_perm(const TabSet& t, cudaStream_t st);
 
 // ---- H x v on column batches (VCA_HAMILTONIAN_SPARSE_HxV.f90:152-200) -----
 // real Hamiltonian, m real columns
