@@ -221,8 +221,8 @@ def hxv_operand(s, D, m, dimup):
         v = s.cfg.hxv_variant
         if m < 16:
             name = "k_hxv_fx"
-        elif v == 2:
-            name = "k_hxv_fx_r"
+        elif v == 2:  # one hopping magnitude here: the packed form from 128 to 1023 up configurations
+            name = "k_hxv_fx_p" if 128 <= dimup <= 1023 else "k_hxv_fx_r"
         elif v == 0 and fits:
             name = "k_hxv_fx_s"
         else:

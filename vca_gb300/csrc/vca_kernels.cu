@@ -358,12 +358,16 @@ __global__ void k_col_dot(int64_t rows, int m, const void* Xv, const void* Yv, d
   }
   if (threadIdx.y == 0 && c < m) partial[(int64_t)blockIdx.x * m + c] = sh[threadIdx.x];
 }
+// A warp a column: one thread adding a column's 608 partials was a chain of as many
+// FP64 additions, 30 us a launch, twice a step (2x2 cluster with 8 bath levels:
+// 20 of 348 ms a solve); 19 and a tree of five give 331 ms.
 __global__ void k_col_reduce(int m, int nblk, const double* partial, double* out) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < m; c += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < nblk; b++) s += partial[(int64_t)b * m + c];
-    out[c] = s;
-  }
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (c >= m) return;  // the whole warp
+  double s = 0.0;
+  for (int b = lane; b < nblk; b += 32) s += partial[(int64_t)b * m + c];
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  if (lane == 0) out[c] = s;
 }
 void launch_col_dot(const ColBatch& b, const void* X, const void* Y, double* partial, int nblk,
                     double* out_col, cudaStream_t st) {
@@ -377,7 +381,7 @@ void launch_col_dot(const ColBatch& b, const void* X, const void* Y, double* par
   else
     k_col_dot<false><<<grd, blk, shm, st>>>(b.rows, b.m, X, Y, partial);
   COUNT_LAUNCH();
-  k_col_reduce<<<nblocks(b.m, 128), 128, 0, st>>>(b.m, nblk, partial, out_col);
+  k_col_reduce<<<(b.m + 3) / 4, 128, 0, st>>>(b.m, nblk, partial, out_col);
 }
 
 template <bool CPLX>
