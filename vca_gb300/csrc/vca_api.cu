@@ -214,6 +214,15 @@ struct Ctx {
     RsShape shape;
     void drop() { ar.release(); slot.clear(); spaces.clear(); tasks.clear(); }
   } rs;
+  // tridiagonals of the batched searches of the current diagonalisation, per sector
+  // (null where it had none): what the eigenvector passes read
+  struct Searched {
+    Arena ar;
+    std::vector<const double*> A, Bt;
+    std::vector<int> steps;
+    void drop() { ar.release(); A.clear(); Bt.clear(); steps.clear(); }
+    bool has(int isector) const { return isector < (int)A.size() && A[isector] && steps[isector] > 0; }
+  } srch;
   int rs_split = 1, rs_diag_im = 0;  // RsParams, of the loaded Hamiltonian
   int ld = 0;
   double* d_poles = nullptr;     // filled on demand from the chain store
@@ -854,8 +863,27 @@ int alloc_batch(Arena& ar, int64_t rows, int m, bool cplx, int nch, int ldab, Ba
 bool resident_sector(int isector);
 int resident_vector(int isector, double* E, void** vec_out, Arena& keep);
 int resident_search(std::vector<double>& energy, const std::vector<char>& run, std::vector<char>& conv);
+
+// Eigenvectors of sectors whose batched search ran: its tridiagonal gives the Ritz
+// pair, and the recurrence is run once more, not twice.  In fixed point every
+// form has the same bits; in FP64 the pass has to repeat the search's own steps
+// (searched_vector: its kernels on the one sector), because coefficients of
+// another order of summation part from the vectors they are used with as the
+// run converges (1e-8 in G' of a BHZ cluster, against 1e-12).  Whole solves: 2x2
+// cluster with 8 bath levels 331 -> 327 ms, 4x3 cluster 772 -> 756 ms.
+int stored_ritz(int isector, double* theta, double* svec, double* resid, double* th) {
+  const Ctx::Searched& T = g->srch;
+  launch_tri_lowest(T.A[isector], T.Bt[isector], T.steps[isector], 0.0, g->cfg.gs_residual_tol, true, theta, svec,
+                    resid, g->st);
+  CUCHK(cudaMemcpyAsync(th, theta, sizeof(double), cudaMemcpyDeviceToHost, g->st));
+  CUCHK(cudaStreamSynchronize(g->st));
+  return VCA_OK;
+}
+int searched_vector(int isector, double* E, void** vec_out, Arena& keep);
+
 int sector_gs(int isector, double* E, void** vec_out, Arena& keep) {
   if (resident_sector(isector)) return resident_vector(isector, E, vec_out, keep);
+  if (g->srch.has(isector)) return searched_vector(isector, E, vec_out, keep);
   const vca_config& c = g->cfg;
   const int nup = sec_nup(isector), ndw = sec_ndw(isector);
   SectorView sv = view_of(nup, ndw);
@@ -891,9 +919,9 @@ int sector_gs(int isector, double* E, void** vec_out, Arena& keep) {
     launch_chain_norm_init(1, bb.meta, norm2, invn, g->st);
     launch_col_scale(cb, invn, X, X, g->st);
   };
-  start(bb.b[0]);
   int mconv = 0;
   double th = 0.0;
+  start(bb.b[0]);
   for (int k = 1; k <= nmax; k++) {
     if ((rc = lanczos_step(sv, cb, bb, k, c.gs_beta_tol, nmax + 1))) { ar.release(); return rc; }
     if (k % std::max(1, c.gs_check_every) == 0 || k == nmax) {
@@ -1141,10 +1169,20 @@ int sector_gs_fx(int isector, double* E, void** vec_out, Arena& keep) {
     launch_chain_norm_init(1, bb.meta, norm2, invn, g->st);
     launch_fx_rescale(cb, invn, 40, fs.F, R, X, bb.scr, g->st);
   };
-  start((i64*)bb.b[0]);
   int mconv = 0;
   double th = 0.0;
-  for (int k = 1; k <= nmax; k++) {
+  const bool stored = g->srch.has(isector);
+  if (stored) {
+    mconv = g->srch.steps[isector];
+    if (!(rc = stored_ritz(isector, theta, svec, resid, &th))) {  // the second pass reads bb.A, bb.Bt
+      cudaMemcpyAsync(bb.A, g->srch.A[isector], sizeof(double) * mconv, cudaMemcpyDeviceToDevice, g->st);
+      cudaMemcpyAsync(bb.Bt, g->srch.Bt[isector], sizeof(double) * mconv, cudaMemcpyDeviceToDevice, g->st);
+    }
+    if (rc) { ar.release(); return rc; }
+  } else {
+    start((i64*)bb.b[0]);
+  }
+  for (int k = 1; !stored && k <= nmax; k++) {
     if ((rc = lanczos_step_fx(sv, fv, cb, bb, k, c.gs_beta_tol, nmax + 1))) { ar.release(); return rc; }
     if (k % std::max(1, c.gs_check_every) == 0 || k == nmax) {
       ChainMeta mh;
@@ -1249,7 +1287,7 @@ int batched_sector_energies(std::vector<double>& energy, const std::vector<char>
         (rc = ar.alloc(&b.X, tot)) || (rc = ar.alloc(&b.Xp, tot)) || (rc = ar.alloc(&b.YW, tot)) ||
         (rc = ar.alloc(&b.tpart, 2 * (size_t)ntiles)) || (rc = ar.alloc(&b.meta, nsec)) ||
         (rc = ar.alloc(&b.alpha, nsec)) || (rc = ar.alloc(&b.bnow, nsec)) ||
-        (rc = ar.alloc(&b.A, (size_t)nsec * ld)) || (rc = ar.alloc(&b.Bt, (size_t)nsec * ld)) ||
+        (rc = g->srch.ar.alloc(&b.A, (size_t)nsec * ld)) || (rc = g->srch.ar.alloc(&b.Bt, (size_t)nsec * ld)) ||
         (rc = ar.alloc(&b.svec, (size_t)nsec * 5 * ld)) || (rc = ar.alloc(&b.theta, nsec)) ||
         (rc = ar.alloc(&b.resid, nsec)) || (rc = ar.alloc(&b.afx, nsec)) || (rc = ar.alloc(&b.bfx, nsec)) ||
         (rc = ar.alloc(&b.mul, nsec)) || (rc = ar.alloc(&b.msh, nsec)) || (rc = ar.alloc(&b.state, nsec)) ||
@@ -1283,12 +1321,23 @@ int batched_sector_energies(std::vector<double>& energy, const std::vector<char>
     }
     CUCHK(cudaGetLastError());
     std::vector<double> th(nsec), rs(nsec);
+    std::vector<int> steps(nsec);
+    cudaMemcpyAsync(steps.data(), b.mconv, sizeof(int) * nsec, cudaMemcpyDeviceToHost, g->st);
     cudaMemcpyAsync(th.data(), b.theta, sizeof(double) * nsec, cudaMemcpyDeviceToHost, g->st);
     cudaMemcpyAsync(rs.data(), b.resid, sizeof(double) * nsec, cudaMemcpyDeviceToHost, g->st);
     CUCHK(cudaStreamSynchronize(g->st));
     for (int q = 0; q < nsec; q++) {
       energy[secs[q].isector - 1] = th[q];
       conv[secs[q].isector - 1] = search_converged(th[q], rs[q]);
+    }
+    Ctx::Searched& T = g->srch;
+    T.A.resize(g->Nsectors + 1, nullptr);
+    T.Bt.resize(g->Nsectors + 1, nullptr);
+    T.steps.resize(g->Nsectors + 1, 0);
+    for (int q = 0; q < nsec; q++) {
+      T.A[secs[q].isector] = b.A + (size_t)q * ld;
+      T.Bt[secs[q].isector] = b.Bt + (size_t)q * ld;
+      T.steps[secs[q].isector] = steps[q];
     }
     ar.release();
     s0 = s1;
@@ -1351,8 +1400,8 @@ int batched_sector_energies_f64(std::vector<double>& energy, const std::vector<c
         (rc = ar.alloc(&x0, (size_t)tot * es)) || (rc = ar.alloc(&x1, (size_t)tot * es)) ||
         (rc = ar.alloc(&x2, (size_t)tot * es)) || (rc = ar.alloc(&b.tpart, ntiles)) ||
         (rc = ar.alloc(&b.meta, nsec)) || (rc = ar.alloc(&b.alpha, nsec)) || (rc = ar.alloc(&b.bnow, nsec)) ||
-        (rc = ar.alloc(&b.invb, nsec)) || (rc = ar.alloc(&b.A, (size_t)nsec * ld)) ||
-        (rc = ar.alloc(&b.Bt, (size_t)nsec * ld)) || (rc = ar.alloc(&b.svec, (size_t)nsec * 5 * ld)) ||
+        (rc = ar.alloc(&b.invb, nsec)) || (rc = g->srch.ar.alloc(&b.A, (size_t)nsec * ld)) ||
+        (rc = g->srch.ar.alloc(&b.Bt, (size_t)nsec * ld)) || (rc = ar.alloc(&b.svec, (size_t)nsec * 5 * ld)) ||
         (rc = ar.alloc(&b.theta, nsec)) || (rc = ar.alloc(&b.resid, nsec)) || (rc = ar.alloc(&b.state, nsec)) ||
         (rc = ar.alloc(&b.mconv, nsec)) || (rc = ar.alloc(&b.undone, 1))) {
       ar.release();
@@ -1387,12 +1436,23 @@ int batched_sector_energies_f64(std::vector<double>& energy, const std::vector<c
     }
     CUCHK(cudaGetLastError());
     std::vector<double> th(nsec), rs(nsec);
+    std::vector<int> steps(nsec);
+    cudaMemcpyAsync(steps.data(), b.mconv, sizeof(int) * nsec, cudaMemcpyDeviceToHost, g->st);
     cudaMemcpyAsync(th.data(), b.theta, sizeof(double) * nsec, cudaMemcpyDeviceToHost, g->st);
     cudaMemcpyAsync(rs.data(), b.resid, sizeof(double) * nsec, cudaMemcpyDeviceToHost, g->st);
     CUCHK(cudaStreamSynchronize(g->st));
     for (int q = 0; q < nsec; q++) {
       energy[secs[q].isector - 1] = th[q];
       conv[secs[q].isector - 1] = search_converged(th[q], rs[q]);
+    }
+    Ctx::Searched& T = g->srch;
+    T.A.resize(g->Nsectors + 1, nullptr);
+    T.Bt.resize(g->Nsectors + 1, nullptr);
+    T.steps.resize(g->Nsectors + 1, 0);
+    for (int q = 0; q < nsec; q++) {
+      T.A[secs[q].isector] = b.A + (size_t)q * ld;
+      T.Bt[secs[q].isector] = b.Bt + (size_t)q * ld;
+      T.steps[secs[q].isector] = steps[q];
     }
     ar.release();
     s0 = s1;
@@ -1837,6 +1897,7 @@ int diagonalize() {
   g->states.release();
   g->gs.clear();
   g->rs.drop();
+  g->srch.drop();
   g->sector_e.assign(g->Nsectors, INFINITY);
   if (c.lanc_method != VCA_LANC_LANCZOS) return g->finiteT ? diagonalize_arpack_finite_t() : diagonalize_arpack_t0();
   if (g->finiteT) return diagonalize_finite_t();
@@ -3344,6 +3405,48 @@ int mt_alloc(MtRun& R, const TaskList& T, int ld, size_t es, bool psi) {
   return VCA_OK;
 }
 
+// The eigenvector of a sector that the FP64 batched search ran: the same steps on
+// the sector by itself (its tiles and their sums are the same), with psi = sum_k s_k x_k.
+int searched_vector(int isector, double* E, void** vec_out, Arena& keep) {
+  const bool cplx = !g->real_model;
+  const size_t es = cplx ? sizeof(double2) : sizeof(double);
+  const int nu = sec_nup(isector), nd = sec_ndw(isector), m = g->srch.steps[isector];
+  const int64_t D = (int64_t)g->dimn[nu] * g->dimn[nd];
+  TaskList V;
+  V.add(view_of(nu, nd), D, isector, 1);
+  MtRun R;
+  const int ld = m + 1;
+  double *svec, *theta, *resid;
+  int* d_m;
+  char* psi;
+  int rc = mt_alloc(R, V, ld, es, true);
+  if (!rc) rc = R.ar.alloc(&svec, 5 * (size_t)ld);
+  if (!rc) rc = R.ar.alloc(&theta, 1);
+  if (!rc) rc = R.ar.alloc(&resid, 1);
+  if (!rc) rc = R.ar.alloc(&d_m, 1);
+  if (!rc) rc = keep.alloc(&psi, (size_t)D * es);
+  if (!rc) rc = stored_ritz(isector, theta, svec, resid, E);
+  if (rc) { R.ar.release(); return rc; }
+  const ChainMeta meta{1, 0, m, 1, 0};
+  cudaMemcpyAsync(d_m, &m, sizeof(int), cudaMemcpyHostToDevice, g->st);
+  cudaMemcpyAsync(R.b.meta, &meta, sizeof(meta), cudaMemcpyHostToDevice, g->st);
+  cudaMemsetAsync(psi, 0, (size_t)D * es, g->st);
+  m64_launch_start(R.gp, cplx, g->cfg.start_seed, R.b, g->st);
+  for (int k = 1; k <= m; k++) {
+    m64_launch_psi(R.gp, cplx, svec, 5 * ld, d_m, k, R.b.X, psi, g->st);
+    if (k < m) m64_launch_step(R.gp, cplx, g->md, k, g->cfg.gs_beta_tol, R.b, g->st);
+  }
+  m64_launch_sqnorm(R.gp, cplx, psi, R.b.tpart, g->st);
+  mt_launch_norm(R.gp, R.b.tpart, R.b.meta, R.n2, R.b.invb, g->st);
+  m64_launch_scale(R.gp, cplx, R.b.invb, psi, psi, g->st);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g->st);
+  R.ar.release();
+  CUCHK(e);
+  *vec_out = psi;
+  return VCA_OK;
+}
+
 // one chain task of the batched form, with the bookkeeping its store needs
 struct BChain {
   int point, state;  // point within the wave, its kept state
@@ -4060,6 +4163,7 @@ int vca_gpu_finalize(void) {
   g->ham.release();
   g->basis.release();
   g->rs.drop();
+  g->srch.drop();
   if (g_pool) {  // every allocation is back
     cudaStreamSynchronize(g_pool_stream);
     cudaMemPoolDestroy(g_pool);
