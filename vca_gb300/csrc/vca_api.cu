@@ -3665,11 +3665,13 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
     const int p1 = p0 + P;
     std::vector<PointTabs> tabs(P);
     std::vector<std::vector<double>> bnd(P);  // per point: lower bound of every sector's energy
+    std::vector<char> mirror(P, 0);           // per point: its spins mirror each other
     bool cplx = false;
     for (int q = 0; q < P; q++) {
       int rc = set_hamiltonian(hl(p0 + q), bh(p0 + q), bv(p0 + q));
       if (rc) { restore(); return rc; }
       if (!c.no_sector_screen) bnd[q] = sector_lower_bounds();
+      mirror[q] = spin_mirror();
       PointTabs& T = tabs[q];
       T.ham.ptrs.swap(g->ham.ptrs);  // the point keeps its tables; set_hamiltonian starts a new arena
       T.sp[0] = g->sp[0];
@@ -3695,12 +3697,14 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
     // upper bound E_up on its ground energy, then only the sectors whose
     // bound lies below E_up + 20 GS_THRESHOLD.  A skipped sector's lowest
     // level is above every level within 20 GS_THRESHOLD of the ground state,
-    // so the T=0 list (VCA_DIAG.f90:224-236) is the one of a full scan.
+    // so the T=0 list (VCA_DIAG.f90:224-236) is the one of a full scan.  Of the
+    // searches left, mirrored ones run once: 2x2 cluster with 8 bath levels, 32
+    // points, search 115 -> 60 ms a point.
     const int LDS = std::min(c.lanc_niter, 512) + 1;  // svec rows kept per (point, sector)
     std::vector<double> theta((size_t)P * nsecs, INFINITY);
     std::vector<int> mconv((size_t)P * nsecs, 0);
     std::vector<double> svec_h((size_t)P * nsecs * LDS, 0.0);
-    std::vector<char> done((size_t)P * nsecs, 0);
+    std::vector<char> done((size_t)P * nsecs, 0), conv((size_t)P * nsecs, 0);
     auto run_search = [&](const std::vector<int>& which /* q * nsecs + (s - 1) */) -> int {
       if (which.empty()) return VCA_OK;
       TaskList S;
@@ -3732,9 +3736,10 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
           if (undone == 0) break;
         }
       }
-      std::vector<double> th(S.secs.size()), sv(S.secs.size() * 5 * (size_t)ldg);
+      std::vector<double> th(S.secs.size()), rs(S.secs.size()), sv(S.secs.size() * 5 * (size_t)ldg);
       std::vector<int> mc(S.secs.size());
       cudaMemcpyAsync(th.data(), R.b.theta, sizeof(double) * th.size(), cudaMemcpyDeviceToHost, g->st);
+      cudaMemcpyAsync(rs.data(), R.b.resid, sizeof(double) * rs.size(), cudaMemcpyDeviceToHost, g->st);
       cudaMemcpyAsync(mc.data(), R.b.mconv, sizeof(int) * mc.size(), cudaMemcpyDeviceToHost, g->st);
       cudaMemcpyAsync(sv.data(), R.b.svec, sizeof(double) * sv.size(), cudaMemcpyDeviceToHost, g->st);
       cudaError_t e = cudaStreamSynchronize(g->st);
@@ -3745,6 +3750,7 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
         theta[t] = th[i];
         mconv[t] = mc[i];
         done[t] = 1;
+        conv[t] = search_converged(th[i], rs[i]);
         const int n = std::min(mc[i], LDS);
         std::copy(sv.begin() + i * 5 * (size_t)ldg, sv.begin() + i * 5 * (size_t)ldg + n,
                   svec_h.begin() + (size_t)t * LDS);
@@ -3752,12 +3758,17 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
       return VCA_OK;
     };
     {
-      std::vector<int> stageA, stageB;
+      // Of two mirrored sectors (spin_mirror) the one with n_up < n_dw waits, and runs
+      // only when its mirror's level is in the window or did not converge.
+      std::vector<int> stageA, stageB, stageC;
+      auto waits = [&](int q, int s2) { return mirror[q] && sec_nup(s2 + 1) < sec_ndw(s2 + 1); };
+      auto at = [&](int q, int s2) { return (size_t)q * nsecs + s2; };
       bool screened = true;
       for (int q = 0; q < P; q++) screened = screened && !bnd[q].empty();
       for (int q = 0; q < P; q++) {
         if (!screened) {
-          for (int s2 = 0; s2 < nsecs; s2++) stageA.push_back(q * nsecs + s2);
+          for (int s2 = 0; s2 < nsecs; s2++)
+            if (!waits(q, s2)) stageA.push_back(q * nsecs + s2);
           continue;
         }
         std::vector<int> ord(nsecs);
@@ -3765,22 +3776,37 @@ int solve_batch_fused(int B, const double* Hloc, int64_t sh, const double* bath_
         std::sort(ord.begin(), ord.end(), [&](int a, int b) { return bnd[q][a] < bnd[q][b]; });
         for (int r = 0; r < std::min(2, nsecs); r++) stageA.push_back(q * nsecs + ord[r]);
       }
+      auto cut = [&](int q) {
+        double e = INFINITY;
+        for (int s2 = 0; s2 < nsecs; s2++)
+          if (done[at(q, s2)]) e = std::min(e, theta[at(q, s2)]);
+        return e + 20.0 * c.gs_threshold + 1e-9 * std::max(1.0, std::fabs(e));
+      };
       int rc = run_search(stageA);
       if (rc) { cleanup(); restore(); return rc; }
+      g->bt_skipped = 0;
       if (screened) {
         for (int q = 0; q < P; q++) {
-          double eup = INFINITY;
-          for (int s2 = 0; s2 < nsecs; s2++)
-            if (done[(size_t)q * nsecs + s2]) eup = std::min(eup, theta[(size_t)q * nsecs + s2]);
-          const double cut = eup + 20.0 * c.gs_threshold + 1e-9 * std::max(1.0, std::fabs(eup));
-          for (int s2 = 0; s2 < nsecs; s2++)
-            if (!done[(size_t)q * nsecs + s2] && !(bnd[q][s2] > cut)) stageB.push_back(q * nsecs + s2);
+          const double top = cut(q);
+          for (int s2 = 0; s2 < nsecs; s2++) {
+            if (done[at(q, s2)]) continue;
+            if (bnd[q][s2] > top) g->bt_skipped++;
+            else if (!waits(q, s2)) stageB.push_back(q * nsecs + s2);
+          }
         }
         rc = run_search(stageB);
         if (rc) { cleanup(); restore(); return rc; }
       }
-      g->bt_skipped = 0;
-      for (char d : done) g->bt_skipped += d ? 0 : 1;
+      for (int q = 0; q < P; q++) {
+        const double top = cut(q);
+        for (int s2 = 0; s2 < nsecs; s2++) {
+          if (done[at(q, s2)] || !waits(q, s2) || (screened && bnd[q][s2] > top)) continue;
+          const size_t m = at(q, sec_of(sec_ndw(s2 + 1), sec_nup(s2 + 1)) - 1);
+          if (!done[m] || !conv[m] || !(theta[m] > top)) stageC.push_back(q * nsecs + s2);
+        }
+      }
+      rc = run_search(stageC);
+      if (rc) { cleanup(); restore(); return rc; }
     }
     lap(1);
     // ---- 3. T=0 lists -------------------------------------------------------
