@@ -1191,7 +1191,9 @@ void launch_recip(int n, const double* in, double* out, cudaStream_t st) {
   COUNT_LAUNCH();
   k_recip<<<nblocks(n, 128), 128, 0, st>>>(n, in, out);
 }
-// (Nlat,Nlat,Nspin,Nspin,Norb,Norb[,L]) -> lso N x N per slice (VCA_AUX_FUNX.f90:255-279)
+// (Nlat,Nlat,Nspin,Nspin,Norb,Norb[,L]) -> lso N x N per slice (VCA_AUX_FUNX.f90:255-279), or
+// back (TO_NNN)
+template <bool TO_NNN>
 __global__ void k_nnn2lso(int Nlat, int Nspin, int Norb, int64_t L, const double2* in, double2* out) {
   const int N = Nlat * Nspin * Norb;
   const int64_t NN = (int64_t)N * N;
@@ -1205,14 +1207,21 @@ __global__ void k_nnn2lso(int Nlat, int Nspin, int Norb, int64_t L, const double
     const int jo = b % Norb, jl = (b / Norb) % Nlat, js = b / (Norb * Nlat);
     const int64_t src = il + (int64_t)Nlat * (jl + (int64_t)Nlat * (is + (int64_t)Nspin *
                         (js + (int64_t)Nspin * (io + (int64_t)Norb * jo))));
-    out[t] = in[l * NN + src];
+    if (TO_NNN) out[l * NN + src] = in[t];
+    else out[t] = in[l * NN + src];
   }
 }
 void launch_nnn2lso(int Nlat, int Nspin, int Norb, int64_t L, const double2* in, double2* out,
                     cudaStream_t st) {
   COUNT_LAUNCH();
   const int N = Nlat * Nspin * Norb;
-  k_nnn2lso<<<nblocks((int64_t)N * N * L, 256), 256, 0, st>>>(Nlat, Nspin, Norb, L, in, out);
+  k_nnn2lso<false><<<nblocks((int64_t)N * N * L, 256), 256, 0, st>>>(Nlat, Nspin, Norb, L, in, out);
+}
+void launch_lso2nnn(int Nlat, int Nspin, int Norb, int64_t L, const double2* in, double2* out,
+                    cudaStream_t st) {
+  COUNT_LAUNCH();
+  const int N = Nlat * Nspin * Norb;
+  k_nnn2lso<true><<<nblocks((int64_t)N * N * L, 256), 256, 0, st>>>(Nlat, Nspin, Norb, L, in, out);
 }
 // P[w] = D[w] + H (lso), or H alone when D == nullptr
 __global__ void k_add_hloc(int nw, int NN, const double2* D, const double2* H, double2* P) {

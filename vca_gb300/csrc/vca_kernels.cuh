@@ -246,6 +246,8 @@ void launch_chain_norm_init(int nch, ChainMeta* meta, const double* norm2, doubl
 void launch_recip(int n, const double* in, double* out, cudaStream_t st);
 void launch_nnn2lso(int Nlat, int Nspin, int Norb, int64_t L, const double2* in, double2* out,
                     cudaStream_t st);
+void launch_lso2nnn(int Nlat, int Nspin, int Norb, int64_t L, const double2* in, double2* out,
+                    cudaStream_t st);
 void launch_add_hloc(int nw, int NN, const double2* D, const double2* H, double2* P, cudaStream_t st);
 void launch_omega_nodes(int n, double scale, const double* s, const double* w, double2* z, double* W,
                         cudaStream_t st);
