@@ -1765,8 +1765,9 @@ void launch_omega_ksum2(int nw, int N, int nblk, int nb, const double2* P, const
 //    largest keeps the elimination stable), their reciprocals are an FP32
 //    estimate and one cubic Newton step (gf_recip);
 //  * the pivots' squared moduli are multiplied up over all k of a thread, as
-//    mantissa and exponent, and so are the 1 + delta of the unpivoted form: a
-//    thread takes a few logarithms at its end instead of one a determinant.
+//    mantissa and exponent, and so are the 1 + delta of the unpivoted form as
+//    long as their product stays near 1 (KluNear): a thread takes a few
+//    logarithms instead of one a determinant.
 // FP64-pipe bound.  BHZ 2x2 (2304 k, 4096 nodes, two 8 x 8 blocks): 121.3 ->
 // 46.1 ms; 4x3 (514 k, 8192 nodes, 12 x 12): 53.4 -> 34.7 ms.
 // ---------------------------------------------------------------------------
@@ -1793,6 +1794,27 @@ struct KluProd {  // prod as mantissa in [1, 2) and exponent
     m = __hiloint2double(hi - (ex << 20), __double2loint(m));
   }
   __device__ __forceinline__ double log_() const { return log(m) + e * 0.6931471805599453; }
+};
+// log of a product of 1 + delta.  Kept as d = product - 1, small deltas lose no
+// digits, but only while d is of order 1: near -1 its digits are gone, and over
+// the k of a mesh whose ln|det| have one sign it would run there or overflow.
+// Out of [-1/2, 1] its logarithm goes to the sum and the product starts again.
+struct KluNear {
+  double d = 0.0;
+  __device__ __forceinline__ static bool near1(double x) { return x >= -0.5 && x <= 1.0; }
+  __device__ __forceinline__ void mul(double delta, double wt, double& acc) {
+    const double t = d + delta + d * delta;
+    if (near1(t)) {
+      d = t;
+      return;
+    }
+    acc = fma(wt, log1p(d), acc);
+    d = delta;
+    if (!near1(delta)) {
+      acc = fma(wt, log1p(delta), acc);
+      d = 0.0;
+    }
+  }
 };
 
 template <int L>
@@ -1830,8 +1852,9 @@ __global__ void __launch_bounds__(KLU_T) k_ksum_lu(int N, int nblk, int nb, int 
   const int nk = (int)(k1 - k0), ntask = nk * nblk;
   double2* a0 = A + slot;
 #define KA(i, j) a0[((i) + (j) * nb) * MT]
-  double acc = 0.0, d1 = 0.0, d2 = 0.0;
-  KluProd p1, p2;
+  double acc = 0.0;
+  KluProd p1, p2;  // of the k-points of weight 1 and 2
+  KluNear d1, d2;
   for (int it = slot; it - slot < ntask; it += MT) {
     const bool valid = it < ntask;
     const int t = valid ? it : ntask - 1;
@@ -1962,9 +1985,9 @@ __global__ void __launch_bounds__(KLU_T) k_ksum_lu(int N, int nblk, int nb, int 
       if (zero) {
         acc = -INFINITY;
       } else if (wt == 1.0) {
-        if (small) d1 = d1 + delta + d1 * delta; else { p1.mul(pt.m); p1.e += pt.e; }
+        if (small) d1.mul(delta, 0.5, acc); else { p1.mul(pt.m); p1.e += pt.e; }
       } else if (wt == 2.0) {
-        if (small) d2 = d2 + delta + d2 * delta; else { p2.mul(pt.m); p2.e += pt.e; }
+        if (small) d2.mul(delta, 1.0, acc); else { p2.mul(pt.m); p2.e += pt.e; }
       } else {
         acc = fma(wt, 0.5 * (small ? log1p(delta) : pt.log_()), acc);
       }
@@ -1972,7 +1995,7 @@ __global__ void __launch_bounds__(KLU_T) k_ksum_lu(int N, int nblk, int nb, int 
     if (L > 1) __syncwarp();
   }
 #undef KA
-  acc += 0.5 * (p1.log_() + log1p(d1)) + (p2.log_() + log1p(d2));
+  acc += 0.5 * (p1.log_() + log1p(d1.d)) + (p2.log_() + log1p(d2.d));
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   __shared__ double red[KLU_T / 32];
   if (lane == 0) red[warp] = acc;
