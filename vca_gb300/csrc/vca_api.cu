@@ -2660,7 +2660,7 @@ int ksum_device(int n, const double2* d_z, bool want_im, Arena& ar, double** f_r
   }
   const int nq = (int)cols.size();
   const double* kw = pairs ? g->d_kw : nullptr;
-  if (!want_im && ksum_lu_ok(N, nblk, nb, nq, pre_m)) {
+  if (!want_im && ksum_lu_ok(N, nblk, nb, nq, pre_m, (int64_t)n * nks * nblk)) {
     std::vector<int> pat(2 * (size_t)nq);  // lso element index; row | col << 8 within the block
     for (int a = 0; a < N; a++)
       for (int q = rowptr[a]; q < rowptr[a + 1]; q++) {

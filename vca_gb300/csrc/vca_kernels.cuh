@@ -195,8 +195,9 @@ void launch_omega_ksum2(int nw, int N, int nblk, int nb, const double2* P, const
                         double* fpart_im, int kchunks, bool pre_m, const KsumInverse& ki, cudaStream_t st);
 // The T=0 integrand (real part) by whole determinants per thread, where
 // ksum_lu_ok: the pattern as nq entries by rows (rowptr), il = their lso element
-// index, ent = row | col << 8 within the block; M as Hk above, Mt: nq*nks scratch
-bool ksum_lu_ok(int N, int nblk, int nb, int nq, bool pre_m);
+// index, ent = row | col << 8 within the block; M as Hk above, Mt: nq*nks scratch;
+// dets: determinants of the call
+bool ksum_lu_ok(int N, int nblk, int nb, int nq, bool pre_m, int64_t dets);
 void launch_ksum_lu(int nw, int N, int nblk, int nb, int nq, const int* il, const int* ent, const int* rowptr,
                     const double2* P, const double2* Glso, int64_t nks, const double2* M, double2* Mt,
                     const double* kw, double* fpart, int kchunks, bool pre_m, const KsumInverse& ki,
