@@ -543,6 +543,12 @@ int vca_gpu_set_chain_streams(int32_t n);
  * VCA_ERR_TIMEOUT.  bytes = 0 (default) restores normal operation.  No
  * counterpart in the reference. */
 int vca_gpu_set_stage_extra_tx(int32_t bytes);
+/* Test hook of a device short of memory: the context behaves as if at most
+ * `bytes` bytes of it were left to it (0, the default: what the device has).
+ * What can be done in parts is; the rest returns VCA_ERR_ALLOC.  Every
+ * allocation waits for the library stream while a limit is set.  No
+ * counterpart in the reference. */
+int vca_gpu_set_memory_limit(int64_t bytes);
 /* The T=0 Omega integrand ln|det(1 + M_k G'(iw))| (VCA_OMEGA.f90:66-67) is
  * evaluated as ln|det(G'^-1 + M_k)| + ln|det G'| at nodes w <= 10, with G'^-1
  * and ln|det G'| formed once per node, which saves the M_k G' product at

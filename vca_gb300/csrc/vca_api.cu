@@ -65,6 +65,14 @@ std::string g_err;
 cudaMemPool_t g_pool = nullptr;
 cudaStream_t g_pool_stream = nullptr;  // the context's stream
 
+uint64_t g_mem_limit = 0;  // most bytes of the pool in use (vca_gpu_set_memory_limit); 0: no limit
+
+// bytes that the limit leaves (the pool's stream is idle)
+uint64_t limit_left() {
+  uint64_t used = 0;
+  cudaMemPoolGetAttribute(g_pool, cudaMemPoolAttrUsedMemCurrent, &used);
+  return used < g_mem_limit ? g_mem_limit - used : 0;
+}
 // free device memory as a budget sees it: what the pool holds unused and
 // above its bound is given back first
 cudaError_t free_memory(size_t* freeb, size_t* totb) {
@@ -73,7 +81,9 @@ cudaError_t free_memory(size_t* freeb, size_t* totb) {
     if (e != cudaSuccess) return e;
     cudaMemPoolTrimTo(g_pool, (size_t)POOL_KEEP);
   }
-  return cudaMemGetInfo(freeb, totb);
+  const cudaError_t e = cudaMemGetInfo(freeb, totb);
+  if (e == cudaSuccess && g_mem_limit) *freeb = std::min<size_t>(*freeb, (size_t)limit_left());
+  return e;
 }
 
 // Device allocations owned by one stage of the context.
@@ -84,8 +94,13 @@ struct Arena {
   int alloc(T** p, size_t n) {
     *p = nullptr;
     if (n == 0) n = 1;
-    cudaError_t e = g_pool ? cudaMallocFromPoolAsync((void**)p, n * sizeof(T), g_pool, st ? st : g_pool_stream)
-                           : cudaMalloc((void**)p, n * sizeof(T));
+    cudaError_t e;
+    if (g_mem_limit && (e = cudaStreamSynchronize(g_pool_stream)) == cudaSuccess && n * sizeof(T) > limit_left())
+      e = cudaErrorMemoryAllocation;
+    else if (g_pool)
+      e = cudaMallocFromPoolAsync((void**)p, n * sizeof(T), g_pool, st ? st : g_pool_stream);
+    else
+      e = cudaMalloc((void**)p, n * sizeof(T));
     if (e != cudaSuccess) {
       *p = nullptr;
       g_err = std::string("cudaMalloc of ") + std::to_string(n * sizeof(T)) + " bytes failed: " +
@@ -1017,8 +1032,23 @@ int resident_launch(int mode, const std::vector<RsSpace>& spaces, const std::vec
   CUCHK(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(RsTask) * tasks.size(), cudaMemcpyHostToDevice, g->st));
   RsParams p{};
   p.spaces = d_spaces;
-  p.tasks = d_tasks;
-  RCHK(ar.alloc(&p.scratch, shape.own * shape.C * tasks.size()));
+  // Scratch is a word for each element of each task of a launch, 41 MB a state of
+  // the 3x3 cluster's chains with two spins.  What the pool keeps between calls is
+  // taken as it is; above that a launch takes the tasks whose scratch fits half of
+  // the free memory, and fewer where that cannot be had.
+  const size_t own = shape.own * shape.C;
+  size_t most = tasks.size();
+  if (own * most * sizeof(i64) > POOL_KEEP) {
+    size_t freeb = 0, totb = 0;
+    CUCHK(free_memory(&freeb, &totb));
+    most = std::max<size_t>(1, std::min(most, freeb / 2 / (own * sizeof(i64))));
+  }
+  int rc;
+  while ((rc = ar.alloc(&p.scratch, own * most)) == VCA_ERR_ALLOC && most > 1) {
+    most = (most + 1) / 2;
+    g_err.clear();
+  }
+  if (rc) return rc;
   p.scratch_block = shape.own;
   p.split = g->rs_split;
   p.diag_im = g->rs_diag_im;
@@ -1030,7 +1060,11 @@ int resident_launch(int mode, const std::vector<RsSpace>& spaces, const std::vec
   p.resid_tol = g->cfg.gs_residual_tol;
   p.check_every = std::max(1, g->cfg.gs_check_every);
   p.mode = mode;
-  if (rs_launch(p, (int)tasks.size(), shape, g->fx ? std::max(1, g->fxbase.K) : 0, !g->real_model, g->st)) CUCHK(cudaGetLastError());
+  for (size_t t = 0; t < tasks.size(); t += most) {  // in stream order, on the same scratch
+    p.tasks = d_tasks + t;
+    const int n = (int)std::min(most, tasks.size() - t);
+    if (rs_launch(p, n, shape, g->fx ? std::max(1, g->fxbase.K) : 0, !g->real_model, g->st)) CUCHK(cudaGetLastError());
+  }
   CUCHK(cudaGetLastError());
   return VCA_OK;
 }
@@ -4195,6 +4229,7 @@ int vca_gpu_finalize(void) {
     cudaMemPoolDestroy(g_pool);
     g_pool = nullptr;
     g_pool_stream = nullptr;
+    g_mem_limit = 0;
   }
   if (g->st) cudaStreamDestroy(g->st);
   if (g->st2) cudaStreamDestroy(g->st2);
@@ -5013,6 +5048,14 @@ int vca_gpu_set_stage_extra_tx(int32_t bytes) {
   if (!g) VFAIL(VCA_ERR_STATE, "vca_gpu_init has not been called");
   if (bytes < 0 || bytes > (1 << 16) || bytes % 16) VFAIL(VCA_ERR_ARG, "0..65536 bytes, a multiple of 16");
   if (fx_set_stage_extra_tx(bytes) != 0) VFAIL(VCA_ERR_CUDA, "cannot set the test hook");
+  return VCA_OK;
+}
+
+int vca_gpu_set_memory_limit(int64_t bytes) {
+  if (!g) VFAIL(VCA_ERR_STATE, "vca_gpu_init has not been called");
+  if (bytes < 0) VFAIL(VCA_ERR_ARG, "bytes must be >= 0");
+  if (!g_pool) VFAIL(VCA_ERR_UNSUPPORTED, "the device has no memory pools");
+  g_mem_limit = (uint64_t)bytes;
   return VCA_OK;
 }
 
