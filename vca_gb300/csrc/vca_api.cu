@@ -4523,8 +4523,6 @@ int vca_gpu_read_gfprime(const char* file, const char* suffix, int32_t used, int
 }
 
 
-// G'(z) at nz host points into the caller's (Nlat,Nlat,Nspin,Nspin,Norb,
-// Norb,nz) array; solve_tables as in gf_lso
 // n lso matrices of the device to the caller's (Nlat,Nlat,Nspin,Nspin,Norb,Norb,n)
 // array, re-ordered on the device in pieces of 16 MB (2000 matrices of the 3x2
 // cluster with two spins: G' 6.1 -> 3.9 ms a call; a loop on the host had
@@ -4535,19 +4533,21 @@ static int lso_to_host(int64_t n, const double2* lso, Arena& ar, double* out) {
   const int64_t piece = std::min<int64_t>(n, std::max<int64_t>(1, ((int64_t)16 << 20) / (NN * (int64_t)sizeof(double2))));
   double2* buf;
   RCHK(ar.alloc(&buf, (size_t)(piece * NN)));
-  // the caller's fresh pages are touched here, while the matrices are still being
+  // the caller's fresh pages are backed here, while the matrices are still being
   // computed: a copy into pages that nothing has written yet is far slower
   // (the same call 10.9 ms)
-  volatile char* page = (volatile char*)out;
-  for (int64_t b = 0; b < n * NN * (int64_t)sizeof(double2); b += 4096) page[b] = 0;
+  touch_pages(out, (size_t)(n * NN) * sizeof(double2));
   for (int64_t q = 0; q < n; q += piece) {
     const int64_t m = std::min(piece, n - q);
     launch_lso2nnn(c.Nlat, c.Nspin, c.Norb, m, lso + q * NN, buf, g->st);
+    CUCHK(cudaGetLastError());
     CUCHK(cudaMemcpyAsync(out + 2 * q * NN, buf, sizeof(double2) * (size_t)(m * NN), cudaMemcpyDeviceToHost, g->st));
   }
   CUCHK(cudaStreamSynchronize(g->st));
   return VCA_OK;
 }
+// G'(z) at nz host points into the caller's (Nlat,Nlat,Nspin,Nspin,Norb,
+// Norb,nz) array; solve_tables as in gf_lso
 static int gf_cluster_host(const double* z, int64_t nz, double* gf_out, bool solve_tables) {
   if (!z || !gf_out || nz < 0) VFAIL(VCA_ERR_ARG, "bad arguments");
   if (nz == 0) return VCA_OK;

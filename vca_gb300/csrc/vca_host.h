@@ -4,6 +4,7 @@
 // them (vca_state_list_t0/_finite_t, vca_pair_kpoints, vca_contour_rule) so
 // that they run without a device.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -41,6 +42,10 @@ bool tridiag_eig(int n, const double* d, const double* e, std::vector<double>& w
 // as columns of Z (column-major n x n, complex interleaved).  Returns false
 // if 100 sweeps did not bring the off-diagonal norm to 1e-15 of the total.
 bool herm_eig(int n, const double* A, std::vector<double>& w, std::vector<double>& Z);
+
+// Has the system back every page of p[0 .. n) with memory, as a first write to it
+// would, and leaves its bytes as they are.
+void touch_pages(void* p, size_t n);
 
 // sets the text vca_gpu_last_error returns and hands the code back
 int set_error(int code, const std::string& msg);
