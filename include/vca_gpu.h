@@ -116,7 +116,11 @@ typedef struct vca_config {
   int32_t sector_at_a_time; /* 1: the ground-state search diagonalises one   */
                            /* sector after the other, as the reference's loop */
                            /* (VCA_DIAG.f90:83-249); 0 (default): every      */
-                           /* sector in one batched search                   */
+                           /* sector in one batched search.  At T=0, where   */
+                           /* the spins mirror each other, a sector with     */
+                           /* n_up < n_dw outside the list's window has its  */
+                           /* mirror's energy in both modes (1: where both   */
+                           /* searches agree within 1e-12)                   */
   double cutoff;           /* CUTOFF     spectrum cut-off exp(-beta dE)      */
   double bandwidth;        /* bandwidth  lattice bandwidth (a module variable */
                            /* the reference's drivers assign, default 0)     */
@@ -522,8 +526,8 @@ int vca_gpu_set_autotune(int32_t on);
  * reads its up hops in an order that pairs the two rows of each quarter
  * warp with sources of opposite parity, so their 16-byte shared-memory
  * reads fall in different banks (on = 1, default); on = 0 keeps the plain
- * sign-sorted order.  Applies to up spaces of 128 configurations and more (the
- * chains of smaller ones run in one launch), when the next Hamiltonian's tables are
+ * sign-sorted order.  Applies to up spaces of 128 configurations and more (in
+ * smaller ones it is worth 1 % at most), when the next Hamiltonian's tables are
  * built; results are bit-identical either way.  No counterpart in the
  * reference. */
 int vca_gpu_set_hop_pairing(int32_t on);
@@ -563,8 +567,11 @@ int vca_gpu_sector_bounds(double* out, int32_t n);
 /* QL sweeps allowed per eigenvalue when the chains' tridiagonals are turned
  * into poles and weights (default 60).
  * A chain that needs more makes the call that asked for poles (the channel
- * getter, the finite-T max_exc, save_gfprime) return VCA_ERR_NUMERIC instead
- * of poles from an unfinished QL.  No counterpart in the reference (SciFortran's
+ * getter, save_gfprime) return VCA_ERR_NUMERIC instead of poles from an
+ * unfinished QL.  max_exc of a finite-T solve needs the largest eigenvalue of
+ * each chain only and finds it without QL; with another limit than 60, with
+ * LANC_NGFITER > 512 or where a chain's numbers are not finite it asks for the
+ * poles, and the solve returns that error.  No counterpart in the reference (SciFortran's
  * eigh stops the process); lowering it makes the failure path testable. */
 int vca_gpu_set_ql_max_iter(int32_t max_iter);
 /* CUDA events on the library stream: device time between start and stop. */

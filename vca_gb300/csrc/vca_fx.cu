@@ -1882,7 +1882,7 @@ static void launch_hxv_fx_s_k(const SectorView& sv, const FxView& fv, int m, con
 #define FXS_DOT_ROWS (152 * 4)  // alpha partial rows of the slab-pair form
 // The down part runs first and writes its half; the up part adds it to its own
 // and, with x and the whole y at hand, forms the <X, Y> sums (apart): they go to
-// row blockIdx % FXS_DOT_ROWS of it (zeroed before) as 128-bit integers in two
+// row rest % FXS_DOT_ROWS of it (zeroed before) as 128-bit integers in two
 // words with the carry of the low one, exact in any order.  16 columns of the
 // 4x4 sector (9,8): 48.5 -> 46.0 ms; with the sums in the down part, which
 // has to read x for them, 51.5.
