@@ -120,6 +120,18 @@ struct Arena {
   }
 };
 
+// A workspace of *most units that does its work in parts just as well: half as
+// many where the allocation fails, down to one.
+template <class T>
+int alloc_most(Arena& ar, T** p, size_t unit, size_t* most) {
+  int rc;
+  while ((rc = ar.alloc(p, unit * *most)) == VCA_ERR_ALLOC && *most > 1) {
+    *most = (*most + 1) / 2;
+    g_err.clear();
+  }
+  return rc;
+}
+
 // Many tables in one allocation, each on a 256-byte boundary.
 struct TableAlloc {
   std::vector<std::pair<char**, size_t>> want;  // where the pointer goes, its offset
@@ -1045,12 +1057,7 @@ int resident_launch(int mode, const std::vector<RsSpace>& spaces, const std::vec
     CUCHK(free_memory(&freeb, &totb));
     most = std::max<size_t>(1, std::min(most, freeb / 2 / (own * sizeof(i64))));
   }
-  int rc;
-  while ((rc = ar.alloc(&p.scratch, own * most)) == VCA_ERR_ALLOC && most > 1) {
-    most = (most + 1) / 2;
-    g_err.clear();
-  }
-  if (rc) return rc;
+  RCHK(alloc_most(ar, &p.scratch, own, &most));
   p.scratch_block = shape.own;
   p.split = g->rs_split;
   p.diag_im = g->rs_diag_im;
@@ -2491,13 +2498,17 @@ int gf_lso(int nz, const double2* d_z, double2* d_Glso, Arena& ar, bool solve_ta
   if (g->gfm_loaded && !solve_tables)
     launch_gf_eval_poles(nelem, g->d_gfm_ptr, g->d_gfm_p, g->d_gfm_w, nz, d_z, raw, g->st);
   else {
-    // in runs of points whose chain values take at most 256 MB
+    // in runs of points whose chain values take at most 256 MB, and fewer where
+    // that cannot be had
     const int nch = g->nstore;
-    const int most = (int)std::max<int64_t>(1, std::min<int64_t>(nz, ((int64_t)1 << 24) / std::max(1, nch)));
+    size_t most = (size_t)std::max<int64_t>(1, std::min<int64_t>(nz, ((int64_t)1 << 24) / std::max(1, nch)));
     double2* val;
-    RCHK(ar.alloc(&val, (size_t)most * nch));
-    for (int q = 0; q < nz; q += most)
-      launch_gf_eval(gf_layout(), nch, std::min(most, nz - q), d_z + q, val, raw + (size_t)q * nelem, g->st);
+    Arena tmp;
+    RCHK(alloc_most(tmp, &val, (size_t)nch, &most));
+    for (int q = 0; q < nz; q += (int)most)
+      launch_gf_eval(gf_layout(), nch, (int)std::min<int64_t>((int64_t)most, nz - q), d_z + q, val,
+                     raw + (size_t)q * nelem, g->st);
+    tmp.release();
   }
   ClusterDims cdm{c.Nlat, c.Norb, c.Nspin, g->N, c.vca_gf_symmetric ? 0 : 1};
   launch_gf_assemble(cdm, nz, raw, d_Glso, g->st);
@@ -2698,16 +2709,22 @@ int ksum_device(int n, const double2* d_z, bool want_im, Arena& ar, double** f_r
   }
   const int nq = (int)cols.size();
   const double* kw = pairs ? g->d_kw : nullptr;
-  if (!want_im && ksum_lu_ok(N, nblk, nb, nq, pre_m, (int64_t)n * nks * nblk)) {
-    std::vector<int> pat(2 * (size_t)nq);  // lso element index; row | col << 8 within the block
+  // pattern entries (lso element index; row | col << 8 within the block) and M
+  // transposed; where there is no room for them the lane groups do without
+  int* d_pat = nullptr;
+  double2* Mt = nullptr;
+  bool lu = !want_im && ksum_lu_ok(N, nblk, nb, nq, pre_m, (int64_t)n * nks * nblk);
+  if (lu && ((rc = ar.alloc(&d_pat, 2 * (size_t)nq)) || (rc = ar.alloc(&Mt, (size_t)nq * nks)))) {
+    g_err.clear();
+    lu = false;
+  }
+  if (lu) {
+    std::vector<int> pat(2 * (size_t)nq);
     for (int a = 0; a < N; a++)
       for (int q = rowptr[a]; q < rowptr[a + 1]; q++) {
         pat[q] = a + cols[q] * N;
         pat[nq + q] = a % nb | (cols[q] % nb) << 8;
       }
-    int* d_pat;
-    double2* Mt;
-    if ((rc = ar.alloc(&d_pat, pat.size())) || (rc = ar.alloc(&Mt, (size_t)nq * nks))) return rc;
     if (nq) CUCHK(cudaMemcpyAsync(d_pat, pat.data(), sizeof(int) * pat.size(), cudaMemcpyHostToDevice, g->st));
     launch_ksum_lu(n, N, nblk, nb, nq, d_pat, d_pat + nq, d_rowptr, P, Glso, nks, hks, Mt, kw, fpart, kchunks, pre_m,
                    ki, g->st);
@@ -4534,15 +4551,15 @@ int vca_gpu_read_gfprime(const char* file, const char* suffix, int32_t used, int
 static int lso_to_host(int64_t n, const double2* lso, Arena& ar, double* out) {
   const vca_config& c = g->cfg;
   const int64_t NN = (int64_t)g->N * g->N;
-  const int64_t piece = std::min<int64_t>(n, std::max<int64_t>(1, ((int64_t)16 << 20) / (NN * (int64_t)sizeof(double2))));
+  size_t piece = (size_t)std::min<int64_t>(n, std::max<int64_t>(1, ((int64_t)16 << 20) / (NN * (int64_t)sizeof(double2))));
   double2* buf;
-  RCHK(ar.alloc(&buf, (size_t)(piece * NN)));
+  RCHK(alloc_most(ar, &buf, (size_t)NN, &piece));
   // the caller's fresh pages are backed here, while the matrices are still being
   // computed: a copy into pages that nothing has written yet is far slower
   // (the same call 10.9 ms)
   touch_pages(out, (size_t)(n * NN) * sizeof(double2));
-  for (int64_t q = 0; q < n; q += piece) {
-    const int64_t m = std::min(piece, n - q);
+  for (int64_t q = 0; q < n; q += (int64_t)piece) {
+    const int64_t m = std::min((int64_t)piece, n - q);
     launch_lso2nnn(c.Nlat, c.Nspin, c.Norb, m, lso + q * NN, buf, g->st);
     CUCHK(cudaGetLastError());
     CUCHK(cudaMemcpyAsync(out + 2 * q * NN, buf, sizeof(double2) * (size_t)(m * NN), cudaMemcpyDeviceToHost, g->st));
