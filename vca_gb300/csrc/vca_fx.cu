@@ -1485,11 +1485,14 @@ __device__ __forceinline__ void fxb_start(uint32_t bar, uint32_t dst, const void
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
-// the CTA's alpha partials: column sums over its rows to row idw of `apart`
-__device__ __forceinline__ void fxr_store_alpha(i128 ad0, i128 ad1, int u, int lane, int warp, int nwarp, int c0, int m,
-                                                int idw, i64* apart) {
+// the CTA's alpha partials: column sums over its rows to row idw of `apart`.  The
+// exchange takes what the CTA's warps need: a fixed 4 KB of it cost L1 (408 columns of
+// the 4x3 sector (6,6) with two hopping magnitudes 7.300 -> 7.255 ms, one 4.009 -> 3.997).
+template <int NWARP>
+__device__ __forceinline__ void fxr_store_alpha(i128 ad0, i128 ad1, int u, int lane, int warp, int c0, int m, int idw,
+                                                i64* apart) {
   constexpr int W = FX_SLAB;
-  __shared__ i128 red[32][W];
+  __shared__ i128 red[NWARP][W];
   i128 adv[2] = {ad0, ad1};
 #pragma unroll
   for (int j = 0; j < 2; j++) {
@@ -1508,7 +1511,7 @@ __device__ __forceinline__ void fxr_store_alpha(i128 ad0, i128 ad1, int u, int l
   __syncthreads();
   if ((int)threadIdx.x < W && c0 + (int)threadIdx.x < m) {
     i128 sum = 0;
-    for (int w = 0; w < nwarp; w++) sum += red[w][threadIdx.x];
+    for (int w = 0; w < NWARP; w++) sum += red[w][threadIdx.x];
     const int64_t o2 = 2 * ((int64_t)idw * m + c0 + threadIdx.x);
     apart[o2] = (i64)(u64)sum;
     apart[o2 + 1] = (i64)(sum >> 64);
@@ -1639,7 +1642,7 @@ __global__ void __launch_bounds__(FXR_THREADS, 4) k_hxv_fx_r(SectorView sv, FxVi
       }
     }
   }
-  if (APART) fxr_store_alpha(ad0, ad1, u, lane, warp, nwarp, c0, m, idw, apart);
+  if (APART) fxr_store_alpha<FXR_THREADS / 32>(ad0, ad1, u, lane, warp, c0, m, idw, apart);
 }
 
 // The same product for one amplitude class (K = 1) with the up hops packed two
@@ -1763,13 +1766,14 @@ __global__ void __launch_bounds__(FXP_THREADS, FXP_BLOCKS) k_hxv_fx_p(SectorView
     }
   }
 #undef FXP_AT
-  if (APART) fxr_store_alpha(ad0, ad1, u, lane, warp, nwarp, c0, m, idw, apart);
+  if (APART) fxr_store_alpha<FXP_THREADS / 32>(ad0, ad1, u, lane, warp, c0, m, idw, apart);
 }
 
 #define FXR_SMEM_MAX (200 * 1024)
 static size_t hxv_fx_r_smem(const SectorView& sv) {
-  return (size_t)(sv.dimup + 1) * FX_SLAB * sizeof(i64) + 16 + (size_t)sv.wdw * 5 + 16;
+  return (size_t)sv.dimup * FX_SLAB * sizeof(i64) + 16 + (size_t)sv.wdw * 5 + 16;
 }
+static size_t hxv_fx_p_smem(const SectorView& sv) { return hxv_fx_r_smem(sv) + FX_SLAB * sizeof(i64); }  // and the zero row
 
 int fx_take_wait_failures() {
   int v = 0;
@@ -1812,7 +1816,7 @@ static void launch_hxv_fx_p_t(const SectorView& sv, const FxView& fv, int m, con
   }
   const int ns = (m + FX_SLAB - 1) / FX_SLAB;
   count_launch_external();
-  k_hxv_fx_p<SH63, APART><<<sv.dimdw * ns, FXP_THREADS, hxv_fx_r_smem(sv), st>>>(sv, fv, m, X, Y, apart);
+  k_hxv_fx_p<SH63, APART><<<sv.dimdw * ns, FXP_THREADS, hxv_fx_p_smem(sv), st>>>(sv, fv, m, X, Y, apart);
 }
 template <int K>
 static void launch_hxv_fx_r_k(const SectorView& sv, const FxView& fv, int m, const i64* X, i64* Y, i64* apart,
