@@ -1487,7 +1487,7 @@ __device__ __forceinline__ void fxb_start(uint32_t bar, uint32_t dst, const void
 }
 // the CTA's alpha partials: column sums over its rows to row idw of `apart`.  The
 // exchange takes what the CTA's warps need: a fixed 4 KB of it cost L1 (408 columns of
-// the 4x3 sector (6,6) with two hopping magnitudes 7.300 -> 7.255 ms, one 4.009 -> 3.997).
+// the 4x3 sector (6,6) with two hopping magnitudes 7.300 -> 7.293 ms, one 4.009 -> 3.997).
 template <int NWARP>
 __device__ __forceinline__ void fxr_store_alpha(i128 ad0, i128 ad1, int u, int lane, int warp, int c0, int m, int idw,
                                                 i64* apart) {
